@@ -71,7 +71,11 @@ typedef enum xcorr_mode {
 /* Kernel families.  The first three mirror the reference's algorithm families; which
  * registry names map to which family is the host program's business. */
 typedef enum xcorr_kernel {
-    XCORR_KERNEL_AUTO = 0,          /* per-shape selection */
+    XCORR_KERNEL_AUTO = 0,          /* per-shape selection: the tile kernel, for a handful of small overlaps the
+                                       warp-per-overlap kernel, and from some tens of microseconds of work on the
+                                       tensor cores (each float as three bfloat16 parts, sums in 32 bits; bit-identical
+                                       from run to run) where those are estimated faster and no less precise.  A
+                                       result may differ from the tile kernel's in its last bits */
     XCORR_KERNEL_TILE = 1,          /* register-tiled circular-class kernel (the fast path) */
     XCORR_KERNEL_OVERLAP_WISE = 2,  /* one thread per overlap -- run_cross_corr_naive_original, naive_original.cu:131-161 */
     XCORR_KERNEL_WARP_PER_OVERLAP = 3, /* one warp per overlap -- run_ccn_warp_per_shift, naive_warp_per_shift.cu:308-335.

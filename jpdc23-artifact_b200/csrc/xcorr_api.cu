@@ -27,8 +27,9 @@ using namespace xcorr;
 // the plan); the text is made when somebody asks for it -- formatting a plan costs about as much
 // host time as enqueuing the kernel of a small input.
 struct LaunchNote {
-    enum Kind { kText, kTile, kStaged, kWarp } kind = kText;
+    enum Kind { kText, kTile, kTensor, kStaged, kWarp } kind = kText;
     TilePlan plan{};
+    TensorPlan tensor{};
     StagedArgs staged{};
     dim3 grid;
     size_t smem = 0;
@@ -566,6 +567,7 @@ xcorr_status plan_tile_search(const PairMap& pm, int H, int W, const xcorr_hints
                                          (2ull * H - 1) * (2ull * W - 1);
     best.workspace_bytes = best.combine == kWorkspace ? (size_t)best.S * total_out * sizeof(float) :
                            best.combine == kFixup ? fixup_counters_offset(best.pieces, total_out) + (size_t)best.tasks * 4 : 0;
+    best.est_us = best_time * 1e6;
     *out = best;
     return XCORR_OK;
 }
@@ -638,6 +640,56 @@ bool tiny_auto(const xcorr_hints* h, const PairMap& pm, uint32_t rows, uint32_t 
     return (double)pm.n_left * pm.m * (2.0 * rows - 1) * (2.0 * cols - 1) <= kTinyOverlaps;
 }
 
+// Whether the automatic choice runs this call on the tensor cores: no hint asks for a plan of another
+// kernel and their estimate beats the tile plan's by a margin.
+bool tensor_auto(const xcorr_hints* h, const PairMap& pm, int H, int W, const DeviceInfo& dev, const TilePlan& tile,
+                 int max_slices, TensorPlan* out) {
+    if (h && (h->kernel != XCORR_KERNEL_AUTO || h->combine || h->overlap_rows || h->class_lanes || h->warps_x ||
+              h->warps_y || h->row_slices || h->schedule || h->block_threads || h->fused_rows))
+        return false;
+    if (dev.smem_optin < (size_t)kSmemLimit) return false;
+    struct Key {
+        uint32_t n_left, m, right_stride;
+        int H, W, sm_count, max_slices;
+        bool operator==(const Key& o) const {
+            return n_left == o.n_left && m == o.m && right_stride == o.right_stride && H == o.H && W == o.W &&
+                   sm_count == o.sm_count && max_slices == o.max_slices;
+        }
+    };
+    struct Entry { Key key; TensorPlan plan; double est_us; };
+    static std::mutex mutex;                       // plans are remembered like the tile kernel's
+    static Entry cache[kPlanCacheSize];
+    static int used = 0, next = 0;
+    const Key k{pm.n_left, pm.m, pm.right_stride, H, W, dev.sm_count, max_slices};
+    Entry e{};
+    bool found = false;
+    {
+        std::lock_guard<std::mutex> lock(mutex);
+        for (int i = 0; i < used && !found; ++i)
+            if (cache[i].key == k) { e = cache[i]; found = true; }
+    }
+    if (!found) {
+        e.key = k;
+        if (!plan_tensor(pm, H, W, dev.sm_count, max_slices, &e.plan, &e.est_us)) e.est_us = 1e30;
+        std::lock_guard<std::mutex> lock(mutex);
+        cache[used < kPlanCacheSize ? used++ : next++ % kPlanCacheSize] = e;
+    }
+    if (!(e.est_us < 0.85 * tile.est_us)) return false;
+    // No less precise than the tile plan.  Error in units of 2^-24 of the result, fitted to 90 measured plans
+    // (uniform operands): a sum of n products taken one after the other is off by 0.185 sqrt(n), and by less
+    // where a plan happens to take it in parts; the tensor cores lose about one unit to rounding towards zero
+    // and 0.2 sqrt(n) to the sums of the rows (87 x 43 61 x 61, cut into 43 parts or more: 1.8 against 2.2;
+    // 64 x 64 1 x 512, in one: 11.8 against 2.0).
+    const double parts = tile.schedule == kSchedStreamK ? std::max(1.0, (double)tile.grid / tile.tasks)
+                       : tile.schedule == kSchedStatic ? (double)tile.S : 1.0;
+    const double sums = (double)H * ((e.plan.Kp + e.plan.KC - 1) / e.plan.KC);
+    const double tile_err2 = 0.0342 * ((double)H * W / (parts * parts) + parts);
+    const double tensor_err2 = 1.0 + 0.04 * (sums / ((double)e.plan.S * e.plan.S) + e.plan.S);
+    if (tensor_err2 > tile_err2) return false;
+    *out = e.plan;
+    return true;
+}
+
 xcorr_status check_sizes(int32_t mode, uint32_t rows, uint32_t cols, uint32_t n_left, uint32_t n_right,
                          PairMap* pm) {
     if (rows == 0 || cols == 0) return fail(XCORR_ERR_INVALID_SIZE, "rows and cols must be positive");
@@ -694,8 +746,20 @@ std::string describe_plan(const TilePlan& p) {
     return buf;
 }
 
+std::string describe_plan(const TensorPlan& p) {
+    char buf[320];
+    std::snprintf(buf, sizeof buf,
+                  "kernel=tensor<%d> grid=(%u,1,1) block=(%d,1,1) smem=%zu tensor{H=%d W=%d side=%s matrices=%d rows=%d interleave=%d x_tiles=%d "
+                  "x_shifts=%d chunk=%d slots=%d S=%d combine=%s}",
+                  p.NC, p.grid, kTensorThreads, p.smem_bytes, p.H, p.W, p.flip ? "right" : "left", p.nB, p.nR, p.J, p.x_tiles, p.DW,
+                  p.KC, p.slots, p.S, p.S > 1 ? "workspace" : "store");
+    return buf;
+}
+
 const std::string& last_launch_text() {
-    if (t_note.kind == LaunchNote::kTile) {
+    if (t_note.kind == LaunchNote::kTensor) {
+        t_last_launch = describe_plan(t_note.tensor);
+    } else if (t_note.kind == LaunchNote::kTile) {
         t_last_launch = describe_plan(t_note.plan);
     } else if (t_note.kind == LaunchNote::kStaged) {
         const StagedArgs& sa = t_note.staged;
@@ -806,6 +870,22 @@ xcorr_status run_device(int32_t mode, const float* d_left, const float* d_right,
         } else if (reinterpret_cast<uintptr_t>(d_ws) % 16 != 0) {
             return fail(XCORR_ERR_WORKSPACE, "workspace must be 16-byte aligned");
         }
+    }
+    TensorPlan tp{};
+    if (tensor_auto(hints, pm, H, W, dev, p, p.combine == kWorkspace ? p.S : 1, &tp)) {
+        TensorArgs ta{};
+        ta.a = tp.flip ? d_right : d_left; ta.b = tp.flip ? d_left : d_right;
+        ta.out = tp.S > 1 ? static_cast<float*>(d_ws) : d_out;
+        ta.slice_floats = total_out;
+        ta.p = tp;
+        t_note.kind = LaunchNote::kTensor; t_note.tensor = tp;
+        XC_CUDA(launch_tensor(ta, device, stream));
+        ++t_launch_count;
+        if (tp.S > 1) {
+            XC_CUDA(launch_reduce_partials(ta.out, d_out, total_out, H, W, H, tp.S, dev.sm_count, stream));
+            ++t_launch_count;
+        }
+        return XCORR_OK;
     }
     TileArgs a{};
     a.left = d_left; a.right = d_right; a.out = d_out;
@@ -1228,6 +1308,11 @@ xcorr_status xcorr_check_device(void) {
         XC_CUDA(cudaGetLastError());
         unsigned timeouts = 0;
         XC_CUDA(tile_stage_timeouts(&timeouts));
+        unsigned tensor_timeouts = 0;
+        XC_CUDA(tensor_wait_timeouts(&tensor_timeouts));
+        if (tensor_timeouts != 0)
+            return fail(XCORR_ERR_TIMEOUT, std::to_string(tensor_timeouts) + " block(s) of tensor_kernel gave up a bounded wait "
+                        "and dropped their work; results of the launches since the last check are incomplete");
         if (timeouts != 0)
             return fail(XCORR_ERR_TIMEOUT, std::to_string(timeouts) + " block(s) of tile_kernel gave up a bounded staging wait "
                         "and dropped their work; results of the launches since the last check are incomplete");
@@ -1286,6 +1371,9 @@ int32_t xcorr_describe_plan(int32_t mode, uint32_t rows, uint32_t cols, uint32_t
         } else {
             if (st != XCORR_OK) return st;
             text = describe_plan(p);
+            TensorPlan tp{};
+            if (tensor_auto(hints, pm, (int)rows, (int)cols, dev, p, p.combine == kWorkspace ? p.S : 1, &tp))
+                text = describe_plan(tp) + "; with tile hints " + text;
         }
     } else {
         return fail(XCORR_ERR_INVALID_HINT, "unknown kernel family");

@@ -10,6 +10,11 @@ namespace xcorr {
 cudaError_t launch_tile(const TileArgs& a, int device, cudaStream_t stream);
 cudaError_t launch_reduce_partials(const float* ws, float* out, unsigned long long total_out,
                                    int H, int W, int Hp, int S, int sm_count, cudaStream_t stream);
+// Tensor cores (xcorr_tensor.cu).  plan_tensor returns false where no plan fits; max_slices > 1 allows
+// row slices with partial images (one matrix on the A side).  *est_us is its estimate of the call.
+bool plan_tensor(const PairMap& pm, int H, int W, int sm_count, int max_slices, TensorPlan* out, double* est_us);
+cudaError_t launch_tensor(const TensorArgs& a, int device, cudaStream_t stream);
+cudaError_t tensor_wait_timeouts(unsigned* count);   // as tile_stage_timeouts
 cudaError_t launch_overlap_wise(const float* left, const float* right, float* out, int H, int W,
                                 PairMap pm, unsigned long long npairs, int block_threads,
                                 dim3* grid_out, dim3* block_out, cudaStream_t stream);

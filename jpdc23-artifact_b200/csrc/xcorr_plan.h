@@ -81,6 +81,7 @@ struct TilePlan {
     unsigned grid;
     size_t smem_bytes;
     size_t workspace_bytes;
+    double est_us;     // the planner's estimate of the call
 };
 
 // Kernel arguments (passed by value).
@@ -121,6 +122,51 @@ struct TileArgs64 {
     TilePlan64 p;
     PairMap pm;
     int vec_ok;        // rows may be fetched two doubles at a time
+};
+
+// Plan and arguments of the tensor-core kernel (xcorr_tensor.cu).
+constexpr int kTensorThreads = 384;
+constexpr int kTensorMaxChunk = 64;   // columns of the A side staged at once, and summed in tensor memory
+constexpr int kTensorMaxSlots = 4;    // Toeplitz rows in flight
+constexpr int kTensorMaxB = 12;       // B matrices of a block
+constexpr int kTensorMaxRow = 576;    // elements of one row of a block's B matrices
+constexpr int kTensorMaxItems = 576;  // 8-element rows of the core matrices of a step
+constexpr int kTensorMaxCols = 128;   // result columns of a drain warp
+constexpr int kTensorMaxJ = 2;        // A matrices interleaved row by row
+constexpr int kTensorMaxStack = 64;   // A matrices a block's rows can touch
+// instruction descriptor without its N: 32-bit accumulators, bfloat16 operands, both K-major, M = 128
+constexpr uint32_t kTensorIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);
+struct TensorPlan {
+    int H, W;
+    int flip;          // 0: A side = left matrices; 1: A side = right matrices (results written mirrored)
+    int nA, nBt;       // matrices of a group on the A side / the B side
+    unsigned groups;   // groups of matrices that meet each other (n_to_mn: one per left)
+    int group_a, group_b, group_pairs;   // matrices of A, of B and results per group
+    int stride_a, stride_b;              // result matrix = group * group_pairs + a * stride_a + b * stride_b
+    int J;             // A matrices interleaved row by row: a stack row is row r of J matrices
+    int stack_rows;    // ceil(nA / J) * H
+    unsigned m_tiles, b_groups;
+    int x_tiles;       // tiles of DW x shifts
+    int DW;            // x shifts of a tile, a multiple of 16
+    int nB;            // B matrices of a block
+    int nR;            // rows of a B matrix taken together (1 or 2)
+    int NC;            // result columns per drain warp: DW * nB * nR <= 2 * NC
+    int Kp, KC;        // padded columns, columns staged at once (multiples of 16)
+    int AR;            // staged rows of the A side (an odd number)
+    int res_rows;      // staged stack rows of one residue mod nR
+    int slots;
+    int row_words;     // 4-byte words of a split row (two elements each), zeros around it included
+    int S;             // slices of B's rows (more than one: partial images)
+    unsigned grid;
+    size_t smem_bytes;
+};
+struct TensorArgs {
+    const float* a;
+    const float* b;
+    float* out;        // the results, or the first partial image
+    int vec_ok;        // A rows may be fetched with 16-byte loads
+    unsigned long long slice_floats;     // floats between partial images
+    TensorPlan p;
 };
 
 // Arguments of the staged warp-per-overlap kernel: a block owns one x shift, `shifts` consecutive

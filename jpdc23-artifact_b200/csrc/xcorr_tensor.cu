@@ -1,0 +1,850 @@
+// Direct cross-correlation on the tensor cores (tcgen05, sm_100a), at single precision.
+//
+// A float is the exact sum of three bfloat16 values, x = h + m + l (8 bits of the significand each),
+// so a product of two floats is nine bfloat16 products; the six that reach 2^-18 of it (hh, hm, mh,
+// hl, mm, lh) are taken and the three below 2^-26 are not.  Bfloat16 products are exact in the
+// tensor cores' 32-bit accumulators.  Those accumulators round towards zero, so no sum stays in them
+// for long: one right row (at most kTensorMaxChunk columns of it) is summed in tensor memory, small
+// products first, and then added to sums in registers, rounded to nearest.
+//
+// As a matrix product.  One side's matrices (the "A side") are stacked to one tall matrix of rows;
+// lane (row of the product) g meets row y of a matrix B of the other side with its row g + y.  Walking
+// y = 0 .. H-1 a lane starts inside matrix g / H at overlap shift sy = g % H and, from y = H - sy on,
+// runs on into the next matrix at shift sy - H (the last one into the first): every product of the
+// cross-correlation is taken exactly once whatever H is, and a wrap costs one write of the lane's sums.
+// The columns of the product are the x shifts: B's row y as a Toeplitz matrix, B[n][k] = row[x0 - n - k].
+// In the unswizzled K-major layout 8 x 8 core matrices may lie anywhere, and a Toeplitz core matrix
+// depends on its block row plus block column alone, so the row needs one core matrix per 8 columns
+// (8 times the row's bytes, written by three producer warps from the row split once) and the two strides
+// of the descriptor are the same.  A step of 16 left columns meets only W + 15 x shifts: the product's N
+// is that window, and its result columns in tensor memory move with it.  What is not taken are the zeros:
+// executed multiply-adds are (W + 15 rounded up to 16) / W of the definition's (1.25 at W = 64), six
+// times over.  A product of N columns takes N / 2 clocks and reads (128 + N) * 32 bytes of shared memory,
+// which yields 128 bytes a clock: below N = 128 the reads would set the pace.  So the columns of several
+// Toeplitz matrices are interleaved in groups of 8 and taken together: of nB matrices B, or, where there
+// are few, of rows y and y - 1 of the same one (nR = 2): lane g then stands for the stack's rows 2 g and
+// 2 g + 1, which meet row y - rho in the same A row 2 g + y, and the A rows are staged even and odd apart.
+//
+// Bound by shared memory: the products alone read it at 75..95 % of its rate, and what the drain warps and the
+// producers move comes on top; a wrapped row costs one to two thousand clocks that two result buffers hide in part.
+// Tried and left: writing a wrapped row from its lane's registers straight to global memory (one 4-byte store in
+// flight per SM every 7 clocks: 64 x 64 1 x 512 took 327 us), 4 and 16 matrices interleaved (fewer wraps, but all
+// warps wait for the one that writes: 32 x 32 32 x 64 88 us against 70).
+// Measured on B200 (us, tile kernel -> this one): 256 x 256 one pair 168 -> 95, 64 x 64 1 x 512 353 -> 119,
+// 32 x 32 32 x 64 101 -> 68, 48 x 48 16 x 2048 450 -> 201, 27 x 43 9 x 35 53 -> 34.
+//
+// Roles of a block (12 warps): warps 0..7 drain tensor memory into register sums and write results,
+// 8..10 build the Toeplitz rows, warp 11 issues the matrix products.
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+#include <algorithm>
+#include <atomic>
+#include <climits>
+#include <cstdint>
+
+#include "xcorr_plan.h"
+#include "xcorr_launch.h"
+
+namespace xcorr {
+
+namespace {
+
+constexpr int kDrainWarps = 8, kProducerWarps = 3;
+constexpr int kMmaWarp = kDrainWarps + kProducerWarps;
+constexpr int kThreads = 32 * (kMmaWarp + 1);
+static_assert(kThreads == kTensorThreads, "block size");
+constexpr int kProducers = 32 * kProducerWarps;
+constexpr int kRowRing = 4;                            // split rows of a B matrix kept by the producers
+constexpr int kRowElems = kTensorMaxRow / kProducers;  // elements of a step's rows per producer thread
+constexpr int kMaxItems = kTensorMaxItems / kProducers;  // Toeplitz rows of a step per producer thread
+constexpr int kMaxSteps = kTensorMaxChunk / 16;
+
+// Operands whose largest magnitude lies outside [2^-60, 2^50) (and infinities and NaN) are not
+// multiplied as three bfloat16 parts: the smallest part of a value below 2^-110 has no bits left, and
+// products of parts must neither overflow nor meet the Toeplitz matrix's zeros as infinities.
+constexpr unsigned kLargeBits = 0x58800000u, kSmallBits = 0x21800000u;
+__device__ __forceinline__ bool out_of_range(unsigned max_bits) {
+    return max_bits >= kLargeBits || (max_bits != 0 && max_bits < kSmallBits);
+}
+
+__device__ unsigned g_tensor_timeouts = 0;
+
+// ---- shared memory, mbarriers, tensor memory ---------------------------------------------------
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void sts128(uint32_t addr, uint4 v) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" :: "r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+__device__ __forceinline__ void bar_init(uint32_t bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool bar_poll(uint32_t bar, uint32_t parity) {
+    unsigned ok;
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// Bounded: false after kStageWaitLimit polls, or once another warp of the block has given up.
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* gave_up) {
+    for (unsigned it = 0; it < kStageWaitLimit; ++it) {
+        if (bar_poll(bar, parity)) return true;
+        if ((it & 63) == 63 && *gave_up) return false;
+    }
+    *gave_up = 1;
+    return false;
+}
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
+}
+__device__ __forceinline__ void tc_mma(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{ .reg .pred p; .reg .b64 a, b;\n\t"
+                 "mov.b64 a, {%1, %3};\n\t"
+                 "mov.b64 b, {%2, %3};\n\t"
+                 "setp.ne.b32 p, %5, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p; }"
+                 :: "r"(d), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
+}
+// Asynchronous: the registers are the caller's after tc_load_wait.
+__device__ __forceinline__ void tc_load(uint32_t addr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(addr));
+}
+// (the registers pass through it, so that nothing reads them earlier)
+__device__ __forceinline__ void tc_load_wait(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :: "memory");
+}
+// Results are written once and never read here; without a memory clobber the compiler may keep the
+// shared-memory loads of the next ones in front.
+__device__ __forceinline__ void put_result(float* to, float v, bool add) {
+    if (add) asm volatile("red.global.add.f32 [%0], %1;" :: "l"(to), "f"(v));
+    else     asm volatile("st.global.f32 [%0], %1;" :: "l"(to), "f"(v));
+}
+__device__ __forceinline__ bool elect_one() {
+    unsigned p;
+    asm volatile("{ .reg .pred p; elect.sync _|p, 0xffffffff; selp.u32 %0, 1, 0, p; }" : "=r"(p));
+    return p != 0;
+}
+
+// Eight floats as three vectors of eight bfloat16: v = h + m + l.
+__device__ __forceinline__ void split8(const float (&v)[8], uint4 (&part)[3]) {
+    uint32_t w[3][4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float a = v[2 * i], b = v[2 * i + 1];
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+            const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
+            w[s][i] = *reinterpret_cast<const uint32_t*>(&p);
+            a -= __uint_as_float(w[s][i] << 16);
+            b -= __uint_as_float(w[s][i] & 0xffff0000u);
+        }
+    }
+#pragma unroll
+    for (int s = 0; s < 3; ++s) part[s] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+}
+
+// One step of 16 columns of the A side: its product's shape, its operands and its place in tensor memory.
+struct Step {
+    uint32_t idesc;      // instruction descriptor with the step's N
+    uint32_t b_off;      // first core matrix of the B operand, in 16-byte units from the part's start
+    uint32_t d_off;      // first result column
+    uint32_t a_off;      // A operand, in 16-byte units from the part's start
+};
+
+struct Shared {
+    unsigned long long b_full[kTensorMaxSlots], b_empty[kTensorMaxSlots], d_full[2], d_empty[2], drained;
+    uint32_t tmem;
+    int gave_up;
+    int n_steps;
+    uint32_t first_off;  // B operand of the chunk's first product, which spans all result columns
+    unsigned bad;
+    unsigned b_max[kTensorMaxB];
+    unsigned a_max[kTensorMaxStack];
+    Step step[kMaxSteps];
+    // a drain warp's columns in the order they are written, neighbours in a result row one after the other
+    // (by Toeplitz matrix, then x shift): column, and its place in its output row's image; INT_MIN: no result
+    int2 column[2 * kTensorMaxCols];
+    long long row_end[2][128];                     // the output rows of a drain lane's last sums
+    long long row_out[2][2][128];                  // a stack row's output rows before / after its wrap, per rho and lane; -1: none
+};
+
+// The block's place in the problem.
+struct BlockTask {
+    const float* a;      // the group's first A matrix
+    const float* b;      // the block's first B matrix
+    float* out;          // the result array, or the slice's partial image
+    long long pair0;     // result matrix of (A matrix 0, the block's first B matrix)
+    int row0;            // first stack row of the block
+    int nb;              // B matrices of this block that exist
+    int sx_lo;           // x shift of column 0
+    int y0, y1;
+};
+
+// The block's results by the definition, straight from global memory: operands that are out of the
+// split's range (see out_of_range).  Eight x shifts of one output row per thread.
+__device__ __noinline__ void direct_block(const TensorArgs& args, const BlockTask t) {
+    const TensorPlan& p = args.p;
+    const int H = p.H, W = p.W, OW = 2 * W - 1, OH = 2 * H - 1;
+    const int groups8 = p.DW / 8 * p.nB;
+    const int total = 128 * p.nR * 2 * groups8;
+    for (int idx = threadIdx.x; idx < total; idx += kThreads) {
+        const int g8 = idx % groups8, row = idx / groups8;
+        const int srow = t.row0 + (row >> 1) / p.J, wrapped = row & 1;
+        const int b = g8 % p.nB, sx0 = t.sx_lo + g8 / p.nB * 8;
+        if (srow >= p.stack_rows || b >= t.nb || sx0 >= W) continue;
+        const int cy = srow % H;
+        int g = srow / H;
+        if (wrapped && (g + 1) * H >= p.stack_rows) g = -1;
+        const int a = (g + wrapped) * p.J + (row >> 1) % p.J;
+        if (a >= p.nA) continue;
+        const int ya = max(t.y0, wrapped ? H - cy : 0), yb = min(t.y1, wrapped ? H : H - cy);
+        if (ya >= yb) continue;
+        const int sy = wrapped ? cy - H : cy;
+        float sum[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) sum[j] = 0.f;
+        for (int y = ya; y < yb; ++y) {
+            const float* ar = t.a + ((size_t)a * H + (y + sy)) * W;
+            const float* br = t.b + ((size_t)b * H + y) * W;
+            for (int u = max(0, sx0); u < min(W, W + sx0 + 7); ++u) {
+                const float av = __ldg(ar + u);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int x = u - sx0 - j;
+                    if (x >= 0 && x < W) sum[j] = fmaf(av, __ldg(br + x), sum[j]);
+                }
+            }
+        }
+        const long long pair = t.pair0 + (long long)a * p.stride_a + (long long)b * p.stride_b;
+        float* o = t.out + pair * ((long long)OH * OW);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int sx = sx0 + j;
+            if (sx >= W) continue;
+            const int at = (sy + H - 1) * OW + sx + W - 1;
+            o[p.flip ? OH * OW - 1 - at : at] = sum[j];
+        }
+    }
+}
+
+// NC: result columns per drain warp (half of the block's).  NR: rows of a B matrix taken together; with
+// two, the 8-column groups belong to row offsets 0 and 1 in turn.
+// MANY: the A side's columns are staged in more than one chunk (a build of its own: the sums then stay in
+// registers across the whole block's code, which the single chunk's warps would pay for with spills).
+template<int NC, int NR, bool MANY>
+__global__ void __launch_bounds__(kThreads, 1) tensor_kernel(const __grid_constant__ TensorArgs args) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ Shared sh;
+    const TensorPlan& p = args.p;
+    const int H = p.H, W = p.W, OW = 2 * W - 1, OH = 2 * H - 1;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    constexpr int D = 2 * NC;                                    // result columns of a buffer
+    constexpr uint32_t kTmemCols = D <= 64 ? 128 : D <= 128 ? 256 : 512;
+
+    // ---- the block's task: x-shift tiles outermost, the heaviest (around shift 0) first
+    BlockTask t;
+    {
+        unsigned id = blockIdx.x;
+        const int slice = (int)(id % p.S); id /= p.S;
+        const int bg = (int)(id % p.b_groups); id /= p.b_groups;
+        const int mt = (int)(id % p.m_tiles); id /= p.m_tiles;
+        const unsigned group = id % p.groups; id /= p.groups;
+        const int order = (int)id, mid = (p.x_tiles - 1) / 2;
+        const int xt = (order & 1) ? mid + (order + 1) / 2 : mid - order / 2;
+        t.row0 = mt * (128 / p.J) * NR;
+        t.nb = min(p.nB, p.nBt - bg * p.nB);
+        t.sx_lo = -(W - 1) + xt * p.DW;
+        t.y0 = (int)((long long)slice * H / p.S);
+        t.y1 = (int)((long long)(slice + 1) * H / p.S);
+        t.a = args.a + (size_t)group * p.group_a * H * W;
+        t.b = args.b + ((size_t)group * p.group_b + (size_t)bg * p.nB) * H * W;
+        t.pair0 = (long long)group * p.group_pairs + (long long)bg * p.nB * p.stride_b;
+        t.out = args.out + (size_t)slice * args.slice_floats;
+    }
+    const int rows = t.y1 - t.y0;
+    const int nS = p.nB * NR;                                              // Toeplitz matrices taken together
+    const int steps_y = rows + NR - 1;                                   // walk of the A side
+    const int n_staged = 128 / p.J * NR + rows - 1;                        // stack rows
+    const int res_rows = p.res_rows;                                     // staged stack rows of one residue mod nR
+
+    const uint32_t a_base = smem_addr(smem);
+    const uint32_t a_part16 = (uint32_t)(p.KC / 8 * p.AR);                 // 16-byte units between the parts of A
+    // (the final write of the results reuses the A side's space, which may have to be larger for it)
+    const uint32_t b_base = a_base + max(3 * a_part16 * 16, (uint32_t)(kDrainWarps * 16 * (NC + 1) * 4));
+    const int n_blk = (p.DW + p.KC) / 8;                                   // core matrices of a Toeplitz row, per B matrix
+    const uint32_t b_part = (uint32_t)(n_blk * nS * 128);
+    const uint32_t slot_bytes = 3 * b_part;
+    const uint32_t ring_base = b_base + p.slots * slot_bytes;              // [part][row mod ring][B matrix][row_words]
+    const uint32_t ring_words = (uint32_t)(kRowRing * p.nB * p.row_words);
+    const int scratch_words = p.J * (NC + 4);
+    float* scratch = reinterpret_cast<float*>(smem + (ring_base - a_base) + 12 * ring_words) + (warp < kDrainWarps ? warp * scratch_words : 0);
+
+    if (tid == 0) {
+        sh.gave_up = 0; sh.bad = 0;
+        for (int i = 0; i < p.slots; ++i) { bar_init(smem_addr(&sh.b_full[i]), kProducers); bar_init(smem_addr(&sh.b_empty[i]), 1); }
+        for (int i = 0; i < 2; ++i) { bar_init(smem_addr(&sh.d_full[i]), 1); bar_init(smem_addr(&sh.d_empty[i]), 32 * kDrainWarps); }
+        bar_init(smem_addr(&sh.drained), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (tid < kTensorMaxB) sh.b_max[tid] = 0;
+    if (tid >= 64 && tid < 64 + kTensorMaxStack) sh.a_max[tid - 64] = 0;
+    // ---- result columns: 8-column groups of the nS Toeplitz matrices in turn
+    for (int c = tid; c < D; c += kThreads) {
+        const int blk = c >> 3, slot = blk % nS, b = slot / NR, n = blk / nS * 8 + (c & 7), sx = t.sx_lo + n;
+        const int first = c / NC * (NC / 8);
+        int before = 0;                            // groups of the same warp written earlier
+        for (int o = first; o < first + NC / 8; ++o) before += o % nS < slot || (o % nS == slot && o < blk);
+        const int at = b * (int)(p.stride_b * ((long long)OH * OW)) + (p.flip ? -(sx + W - 1) : sx + W - 1);
+        sh.column[c / NC * NC + before * 8 + (c & 7)] = make_int2(c % NC, n < p.DW && b < t.nb && sx < W ? at : INT_MIN);
+    }
+    if (warp == kMmaWarp) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_addr(&sh.tmem)), "r"(kTmemCols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = sh.tmem;
+
+    // ---- largest magnitude of every B matrix of the block (the slice's rows)
+    for (int b = 0; b < t.nb; ++b) {
+        const unsigned* src = reinterpret_cast<const unsigned*>(t.b + ((size_t)b * H + t.y0) * W);
+        unsigned mx = 0;
+        for (int i = tid; i < rows * W; i += kThreads) mx = max(mx, __ldg(src + i) & 0x7fffffffu);
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        if (lane == 0) atomicMax(&sh.b_max[b], mx);
+    }
+
+    // ---- the lanes' output rows
+    const int half_col = (warp >> 2) * NC;
+    // first element of the output row of matrix j of a stack row's group, for its shift before (0) or after (1)
+    // the wrap; -1: no such matrix
+    auto row_offset = [&](int srow, int j, int wrapped) -> long long {
+        int g = srow / H;
+        const int sy = srow - g * H - (wrapped ? H : 0);
+        if (wrapped) g = (g + 1) * H < p.stack_rows ? g + 1 : 0;
+        const int a = g * p.J + j, at = (sy + H - 1) * OW;
+        if (srow >= p.stack_rows || a >= p.nA) return -1;
+        return (t.pair0 + (long long)a * p.stride_a) * ((long long)OH * OW) + (p.flip ? OH * OW - 1 - at : at);
+    };
+    bool wrapped[NR];                              // the sums at hand belong to the shift after the wrap
+    int wrap_step[NR];                             // step with which a drain lane's rows run on into the next group; -1: never
+#pragma unroll
+    for (int rho = 0; rho < NR; ++rho) {
+        const int m = (warp & 3) * 32 + lane, srow = t.row0 + m / p.J * NR + rho, y = H - srow % H;
+        wrap_step[rho] = srow < p.stack_rows && y > t.y0 && y < t.y1 ? y - t.y0 + rho : -1;
+        if (warp < 4) {
+            sh.row_out[0][rho][m] = row_offset(srow, m % p.J, 0);
+            sh.row_out[1][rho][m] = row_offset(srow, m % p.J, 1);
+        }
+        wrapped[rho] = y <= t.y0;
+    }
+
+    unsigned it_base = 0;                          // rows walked before the current chunk
+    int pass = 0;                                  // chunks walked
+    // The chunks are walked to and fro: a stack row that does not wrap on the way keeps its sums from chunk
+    // to chunk, one that does writes them at its turning point once per chunk (added from the third time on).
+    float sum[NC];
+    if (MANY) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) sum[c] = 0.f;
+    }
+    bool ok = true;
+    for (int k0 = 0; k0 < p.Kp; k0 += p.KC) {
+        const int kc = min(p.KC, p.Kp - k0);
+        const int X0 = p.Kp - 1 - t.sx_lo - k0;    // column of B that chunk column k meets at result column n: X0 - n - k
+        // steps that meet the tile's x shifts at all; uniform over the block
+        int any = 0;
+        for (int s = 0; s < kc / 16; ++s) {
+            const int lo = max(0, (X0 - W + 1 - 16 * s - 15) & ~7), hi = min(p.DW, X0 - 16 * s + 1);
+            any |= hi > lo;
+        }
+        if (!any) continue;
+
+        // ---- stage the chunk: A rows as three parts, zeros into the Toeplitz slots, the step table
+        {
+            // (neighbouring threads take neighbouring columns; an odd AR spreads their stores over the banks)
+            const int kq = kc / 8, items = n_staged * p.J * kq;
+            const uint32_t kq_rcp = (65536u + kq - 1) / kq;             // exact for the few thousand items there are
+            const int first_row = t.row0 + t.y0;
+            for (int i0 = 0; i0 < items; i0 += kThreads) {
+                const int i = min(i0 + tid, items - 1);                 // (the last items again rather than idle lanes)
+                const int r = (int)(((uint32_t)i * kq_rcp) >> 16), q = i - r * kq;
+                const int sr = r / p.J, j = r - sr * p.J;
+                int srow = first_row + sr;                              // (the stack starts over behind its end)
+                while (srow >= p.stack_rows) srow -= p.stack_rows;
+                const int g = srow / H, mat = g * p.J + j, local = (t.row0 % H + t.y0 + sr) / H * p.J + j;
+                const bool there = mat < p.nA;
+                const float* src = t.a + ((size_t)(there ? mat : 0) * H + (srow - g * H)) * W;
+                const int u0 = p.Kp - 8 - (k0 + q * 8);                 // the item's columns: u0 + 7 down to u0
+                float v[8];
+                if (args.vec_ok && u0 + 8 <= W) {
+                    const float4 lo = __ldg(reinterpret_cast<const float4*>(src + u0)), hi = __ldg(reinterpret_cast<const float4*>(src + u0 + 4));
+                    v[0] = hi.w; v[1] = hi.z; v[2] = hi.y; v[3] = hi.x; v[4] = lo.w; v[5] = lo.z; v[6] = lo.y; v[7] = lo.x;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) v[k] = there && u0 + 7 - k < W ? __ldg(src + u0 + 7 - k) : 0.f;
+                }
+                unsigned mx = 0;
+#pragma unroll
+                for (int k = 0; k < 8; ++k) mx = max(mx, __float_as_uint(v[k]) & 0x7fffffffu);
+                if (there) atomicMax(&sh.a_max[local], mx);
+                uint4 part[3];
+                split8(v, part);
+                const uint32_t at = a_base + (uint32_t)(q * p.AR + ((sr % NR) * res_rows + sr / NR) * p.J + j) * 16;
+#pragma unroll
+                for (int s = 0; s < 3; ++s) sts128(at + s * a_part16 * 16, part[s]);
+            }
+            for (uint32_t i = tid * 16; i < p.slots * slot_bytes + 12 * ring_words; i += kThreads * 16) sts128(b_base + i, make_uint4(0, 0, 0, 0));
+            if (tid == 0) {
+                int n = 0;
+                for (int s = 0; s < kc / 16; ++s) {
+                    int lo = max(0, (X0 - W + 1 - 16 * s - 15) & ~7);
+                    const int hi = min(p.DW, X0 - 16 * s + 1);
+                    if (hi <= lo) continue;
+                    const int cols = (hi - lo + 15) & ~15;
+                    if (lo + cols > p.DW) lo = p.DW - cols;
+                    Step st;
+                    st.idesc = kTensorIdesc | (uint32_t)(cols * nS / 8) << 17;
+                    st.b_off = (uint32_t)((2 * s + lo / 8) * nS * 8);
+                    st.d_off = (uint32_t)(lo * nS);
+                    st.a_off = (uint32_t)(2 * s * p.AR);
+                    if (n == 0) sh.first_off = (uint32_t)(2 * s * nS * 8);
+                    sh.step[n++] = st;
+                }
+                sh.n_steps = n;
+            }
+            fence_async();
+            __syncthreads();
+        }
+
+        const int back = MANY ? pass & 1 : 0;
+        if (warp < kDrainWarps) {
+            // ================= drain: tensor memory -> register sums -> results
+            if (!MANY) {
+#pragma unroll
+                for (int c = 0; c < NC; ++c) sum[c] = 0.f;
+            }
+            const uint32_t t_addr = tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)half_col;
+            for (int i = 0; ok && i < steps_y; ++i) {
+                const unsigned it = it_base + i;
+                // stack rows that run on into the next matrices with this step: their sums so far are result
+                // rows, written by the whole warp (J lanes wrap at a time), and the next sums start from zero
+                const int turn = back ? steps_y - i : i;       // (backwards, the rows come back with the step before)
+                const unsigned who0 = __ballot_sync(0xffffffffu, turn == wrap_step[0]);
+                const unsigned who1 = NR == 2 ? __ballot_sync(0xffffffffu, turn == wrap_step[NR - 1]) : 0u;
+                const unsigned who = who0 | who1;
+                const float keep0 = who0 >> lane & 1 ? 0.f : 1.f, keep1 = who1 >> lane & 1 ? 0.f : 1.f;
+                if (who0 >> lane & 1) wrapped[0] = !back;
+                if (NR == 2 && (who1 >> lane & 1)) wrapped[NR - 1] = !back;
+                for (unsigned rest = who; rest;) {
+                    // (more than one group of J lanes where a warp's stack rows span more than H)
+                    const unsigned group = ((1u << p.J) - 1u) << ((__ffs(rest) - 1) & ~(p.J - 1)), now = rest & group;
+                    rest &= ~group;
+                    if (now >> lane & 1) {
+                        float4* to = reinterpret_cast<float4*>(scratch + lane % p.J * (NC + 4));
+#pragma unroll
+                        for (int c = 0; c < NC; c += 4) to[c / 4] = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
+                    }
+                    __syncwarp();
+                    // (with two rows taken together the first half of the order belongs to row offset 0)
+                    const int2* column = &sh.column[half_col + lane];
+                    int2 col[NC / 32];
+#pragma unroll
+                    for (int z = 0; z < NC / 32; ++z) col[z] = column[32 * z];
+                    for (unsigned left = now; left; left &= left - 1) {
+                        const int src = __ffs(left) - 1;
+                        const float* from = scratch + src % p.J * (NC + 4);
+                        const long long off0 = who0 >> src & 1 ? sh.row_out[back][0][(warp & 3) * 32 + src] : -1;
+                        const long long off1 = NR == 2 && (who1 >> src & 1) ? sh.row_out[back][NR - 1][(warp & 3) * 32 + src] : -1;
+                        float v[NC / 32];
+#pragma unroll
+                        for (int z = 0; z < NC / 32; ++z) v[z] = from[col[z].x];
+#pragma unroll
+                        for (int z = 0; z < NC / 32; ++z) {
+                            const long long off = NR == 2 && 32 * z + lane >= NC / 2 ? off1 : off0;
+                            if (off >= 0 && col[z].y != INT_MIN) put_result(t.out + off + col[z].y, v[z], MANY && pass >= 2);
+                        }
+                    }
+                    __syncwarp();
+                }
+                ok = bar_wait(smem_addr(&sh.d_full[it & 1]), (it >> 1) & 1, &sh.gave_up);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll
+                for (int c0 = 0; c0 < NC; c0 += 16) {
+                    uint32_t v[16];
+                    tc_load(t_addr + (it & 1) * D + c0, v);
+                    tc_load_wait(v);
+                    if (c0 + 16 >= NC) { tc_fence_before(); bar_arrive(smem_addr(&sh.d_empty[it & 1])); }
+#pragma unroll
+                    for (int c = 0; c < 16; ++c)
+                        sum[c0 + c] = fmaf(sum[c0 + c], NR == 2 && (c & 8) ? keep1 : keep0, __uint_as_float(v[c]));   // (exact: times 1 or 0)
+                }
+            }
+        } else if (warp < kMmaWarp) {
+            // ================= producers: row y of every B matrix of the block as a Toeplitz matrix
+            // A row is split once and kept reversed as three runs of bfloat16 (element e is column X0 - e);
+            // row n of core matrix i is the eight elements from e = 8 i + n on.
+            const int ptid = tid - 32 * kDrainWarps;
+            const int i_lo = max(0, (X0 - W + 1 - 14 + 7) >> 3), i_hi = min(n_blk - 1, X0 >> 3);
+            const int items = max(0, i_hi - i_lo + 1) * nS * 8, row_elems = t.nb * W;
+            const int e_end = 8 * (i_hi - i_lo + 1) + 8;
+            const uint32_t part_bytes = 4 * ring_words, row_bytes = (uint32_t)p.row_words * 4;
+            float ahead[kRowElems];
+            uint32_t at[kRowElems];               // byte offset of the element in a ring row set; ~0: not needed
+            const float* from[kRowElems];
+#pragma unroll
+            for (int j = 0; j < kRowElems; ++j) {
+                const int idx = ptid + j * kProducers, b = idx / W, x = idx - b * W;
+                const int e = X0 - x - 8 * i_lo;
+                at[j] = idx < row_elems && e >= 0 && e < e_end ? (uint32_t)b * row_bytes + 2u * (uint32_t)e : ~0u;
+                from[j] = t.b + ((size_t)b * H + t.y0) * W + x;
+                if (back) from[j] += (size_t)(rows - 1) * W;
+                ahead[j] = at[j] != ~0u ? __ldg(from[j]) : 0.f;
+            }
+            // the thread's Toeplitz rows: where they are read in a ring row and written in a slot
+            uint32_t item[kMaxItems], item_dst[kMaxItems];
+#pragma unroll
+            for (int j = 0; j < kMaxItems; ++j) {
+                const int e = ptid + j * kProducers, n = e & 7, blk = e >> 3, bi = blk / nS, sl = blk - bi * nS, b = sl / NR;
+                item[j] = (uint32_t)b * row_bytes + (uint32_t)(4 * bi + (n >> 1)) * 4 + (NR == 2 ? (uint32_t)(sl & 1) << 31 : 0u);
+                item_dst[j] = (uint32_t)((i_lo * nS + blk) * 128 + n * 16);
+            }
+            const uint32_t shift = (ptid & 1) * 16;
+            // (a warp that gave up a wait keeps meeting the others at the barrier)
+            for (int i = 0; i < steps_y; ++i) {
+                const unsigned it = it_base + i, use = it / p.slots;
+                const int slot = (int)(it - use * p.slots);
+                // step's place in the walk, and the row it brings: the first of its rows, or backwards the last
+                const int place = back ? steps_y - 1 - i : i, fresh = back ? place - (NR - 1) : place;
+                const uint32_t ring_row = ring_base + (uint32_t)(fresh & (kRowRing - 1)) * (uint32_t)p.nB * row_bytes;
+                const bool real = fresh >= 0 && fresh < rows;
+#pragma unroll
+                for (int j = 0; j < kRowElems; ++j) {
+                    if (at[j] == ~0u) continue;
+                    float v = real ? ahead[j] : 0.f;              // (beyond the first and last row: zeros)
+#pragma unroll
+                    for (int s = 0; s < 3; ++s) {
+                        const __nv_bfloat16 h = __float2bfloat16_rn(v);
+                        asm volatile("st.shared.b16 [%0], %1;" :: "r"(ring_row + at[j] + s * part_bytes),
+                                     "h"(__bfloat16_as_ushort(h)) : "memory");
+                        v -= __bfloat162float(h);
+                    }
+                    if (i + 1 < rows) ahead[j] = __ldg(from[j] + (back ? -(long long)(i + 1) * W : (long long)(i + 1) * W));
+                }
+                asm volatile("bar.sync 1, %0;" :: "n"(kProducers) : "memory");
+                if (ok && use > 0) ok = bar_wait(smem_addr(&sh.b_empty[slot]), (use - 1) & 1, &sh.gave_up);
+                ok = __all_sync(0xffffffffu, ok);
+                const uint32_t dst0 = b_base + slot * slot_bytes, set_bytes = (uint32_t)p.nB * row_bytes;
+                const uint32_t src0 = ring_base + (uint32_t)(place & (kRowRing - 1)) * set_bytes;
+                const uint32_t src1 = ring_base + (uint32_t)((place - 1) & (kRowRing - 1)) * set_bytes;
+                if (ok) {
+#pragma unroll
+                    for (int j = 0; j < kMaxItems; ++j) {
+                        if (j * kProducers >= items) break;
+                        if (ptid + j * kProducers >= items) continue;
+                        const uint32_t src = NR == 2 ? ((int)item[j] < 0 ? src1 : src0) + (item[j] & 0x7fffffffu) : src0 + item[j];
+                        uint32_t w[3][5];
+#pragma unroll
+                        for (int s = 0; s < 3; ++s)
+#pragma unroll
+                            for (int k = 0; k < 5; ++k)
+                                asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w[s][k]) : "r"(src + s * part_bytes + 4 * k));
+#pragma unroll
+                        for (int s = 0; s < 3; ++s)
+                            sts128(dst0 + item_dst[j] + s * b_part,
+                                   make_uint4(__funnelshift_r(w[s][0], w[s][1], shift), __funnelshift_r(w[s][1], w[s][2], shift),
+                                              __funnelshift_r(w[s][2], w[s][3], shift), __funnelshift_r(w[s][3], w[s][4], shift)));
+                    }
+                }
+                fence_async();
+                bar_arrive(smem_addr(&sh.b_full[slot]));
+            }
+        } else {
+            // ================= matrix products: one row of B against 128 rows of A
+            const bool leader = elect_one();
+            const uint32_t desc_hi = 8u | 1u << 14;                       // 128 bytes between groups of 8 rows; descriptor version
+            const uint32_t a_lo0 = (a_base >> 4) | (uint32_t)p.AR << 16, lbo_b = (uint32_t)(8 * nS) << 16;
+            const uint32_t idesc_all = kTensorIdesc | (uint32_t)(p.DW * nS / 8) << 17;
+            const uint32_t bp = b_part >> 4, first_off = sh.first_off;
+            const int n_steps = sh.n_steps;
+            Step st[kMaxSteps];
+#pragma unroll
+            for (int s = 0; s < kMaxSteps; ++s) st[s] = sh.step[s < n_steps ? s : 0];
+            for (int i = 0; ok && i < steps_y; ++i) {
+                const unsigned it = it_base + i, use = it / p.slots;
+                const int slot = (int)(it - use * p.slots);
+                ok = bar_wait(smem_addr(&sh.b_full[slot]), use & 1, &sh.gave_up);
+                if (ok && it >= 2) ok = bar_wait(smem_addr(&sh.d_empty[it & 1]), ((it >> 1) - 1) & 1, &sh.gave_up);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after();
+                if (leader) {
+                    const int place = back ? steps_y - 1 - i : i;
+                    const uint32_t a0 = a_lo0 + ((place % NR) * res_rows + place / NR) * p.J, d0 = tmem + (it & 1) * D;
+                    const uint32_t b0 = ((b_base + slot * slot_bytes) >> 4) | lbo_b;
+                    // the products of the small parts first: they lose nothing beside the sum of the large ones.
+                    // The row's first product spans all result columns (against the Toeplitz matrix's zeros
+                    // outside its window) and overwrites the buffer.
+                    tc_mma(d0, a0 + st[0].a_off + 2 * a_part16, b0 + first_off, desc_hi, idesc_all, 0);
+#pragma unroll
+                    for (int s = 0; s < kMaxSteps; ++s) {
+                        if (s >= n_steps) break;
+                        const uint32_t a = a0 + st[s].a_off, b = b0 + st[s].b_off, d = d0 + st[s].d_off, id = st[s].idesc;
+                        if (s > 0) tc_mma(d, a + 2 * a_part16, b, desc_hi, id, 1);
+                        tc_mma(d, a, b + 2 * bp, desc_hi, id, 1);
+                        tc_mma(d, a + a_part16, b + bp, desc_hi, id, 1);
+                        tc_mma(d, a + a_part16, b, desc_hi, id, 1);
+                        tc_mma(d, a, b + bp, desc_hi, id, 1);
+                    }
+#pragma unroll
+                    for (int s = 0; s < kMaxSteps; ++s) {
+                        if (s >= n_steps) break;
+                        tc_mma(d0 + st[s].d_off, a0 + st[s].a_off, b0 + st[s].b_off, desc_hi, st[s].idesc, 1);
+                    }
+                    tc_commit(smem_addr(&sh.b_empty[slot]));
+                    tc_commit(smem_addr(&sh.d_full[it & 1]));
+                }
+                __syncwarp();
+            }
+        }
+        it_base += steps_y;
+        ++pass;
+        tc_fence_before();
+        if (__syncthreads_or(!ok)) { ok = false; break; }
+        tc_fence_after();
+        if (!MANY) break;
+    }
+
+    // ---- the walk's end: all sums are result rows.  Through shared memory (the A side is done with: all
+    // products have completed), 16 lanes at a time, so that a store instruction writes up to 32 neighbours.
+    if (ok && warp < kDrainWarps) {
+        float* tile = reinterpret_cast<float*>(smem) + warp * 16 * (NC + 1);
+        // (both halves of a warp's columns set the same values)
+        unsigned again[NR];                        // rows that wrapped on the way have been written before, unless this was the only pass
+#pragma unroll
+        for (int rho = 0; rho < NR; ++rho) {
+            again[rho] = MANY && pass > 1 ? __ballot_sync(0xffffffffu, wrap_step[rho] >= 0) : 0u;
+            sh.row_end[rho][(warp & 3) * 32 + lane] = sh.row_out[wrapped[rho] ? 1 : 0][rho][(warp & 3) * 32 + lane];
+        }
+#pragma unroll 1
+        for (int half = 0; half < 2; ++half) {
+            if (lane >> 4 == half) {
+#pragma unroll
+                for (int c = 0; c < NC; ++c) tile[(lane & 15) * (NC + 1) + c] = sum[c];
+            }
+            __syncwarp();
+#pragma unroll 1
+            for (int z = 0; z < NC / 32; ++z) {
+                const int2 col = sh.column[half_col + 32 * z + lane];
+                if (col.y != INT_MIN) {
+                    const bool second = NR == 2 && 32 * z + lane >= NC / 2;
+                    const long long* offs = &sh.row_end[second ? 1 : 0][(warp & 3) * 32 + half * 16];
+                    const unsigned ag = MANY ? again[second ? NR - 1 : 0] >> (half * 16) : 0u;
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) {
+                        const long long off = offs[r];
+                        const float v = tile[r * (NC + 1) + col.x];
+                        if (off >= 0) put_result(t.out + off + col.y, v, ag >> r & 1);
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+
+    // ---- operands the split does not cover: the block's results again, by the definition
+    if (tid < kTensorMaxStack && out_of_range(sh.a_max[tid])) sh.bad = 1;
+    if (tid < t.nb && out_of_range(sh.b_max[tid])) sh.bad = 1;
+    __syncthreads();
+    if (warp == kMmaWarp) {
+        if (!ok) {
+            // products may be in flight: let them land before their memory goes
+            if (elect_one()) tc_commit(smem_addr(&sh.drained));
+            __syncwarp();
+            for (unsigned it = 0; it < kStageWaitLimit && !bar_poll(smem_addr(&sh.drained), 0); ++it) {}
+            __syncwarp();
+        }
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(kTmemCols) : "memory");
+    }
+    if (!ok) {
+        if (tid == 0) atomicAdd(&g_tensor_timeouts, 1u);
+        return;
+    }
+    if (sh.bad) {
+        direct_block(args, t);
+        return;
+    }
+    // ---- the corners of a result are single products: rounded once, as the definition has them (the three
+    // products of parts left out and the rounding towards zero would show in their last bit)
+    for (int i = tid; i < 128 * NR * t.nb * 2; i += kThreads) {
+        const int right_side = i & 1, b = (i >> 1) % t.nb, m = (i >> 1) / t.nb;
+        const int srow = t.row0 + m / p.J, cy = srow % H, sx = right_side ? W - 1 : 1 - W;
+        if (srow >= p.stack_rows || sx < t.sx_lo || sx >= t.sx_lo + p.DW) continue;
+        int g = srow / H;
+        const bool bottom = cy == H - 1 && t.y0 == 0, top = cy == 1 && t.y1 == H;       // shift H - 1 / 1 - H
+        if (!bottom && !top) continue;
+        if (top) g = (g + 1) * H < p.stack_rows ? g + 1 : 0;
+        const int a = g * p.J + m % p.J;
+        if (a >= p.nA) continue;
+        const float av = __ldg(t.a + ((size_t)a * H + (bottom ? H - 1 : 0)) * W + (right_side ? W - 1 : 0));
+        const float bv = __ldg(t.b + ((size_t)b * H + (bottom ? 0 : H - 1)) * W + (right_side ? 0 : W - 1));
+        const int at = (bottom ? OH - 1 : 0) * OW + (right_side ? OW - 1 : 0);
+        const long long pair = t.pair0 + (long long)a * p.stride_a + (long long)b * p.stride_b;
+        t.out[pair * ((long long)OH * OW) + (p.flip ? OH * OW - 1 - at : at)] = av * bv;
+    }
+}
+
+int up(int v, int m) { return (v + m - 1) / m * m; }
+
+}  // namespace
+
+cudaError_t launch_tensor(const TensorArgs& a, int device, cudaStream_t stream) {
+    void (*const kernels[2][2][4])(TensorArgs) = {
+        {{tensor_kernel<32, 1, false>, tensor_kernel<64, 1, false>, tensor_kernel<96, 1, false>, tensor_kernel<128, 1, false>},
+         {tensor_kernel<32, 1, true>, tensor_kernel<64, 1, true>, tensor_kernel<96, 1, true>, tensor_kernel<128, 1, true>}},
+        {{tensor_kernel<32, 2, false>, tensor_kernel<64, 2, false>, tensor_kernel<96, 2, false>, tensor_kernel<128, 2, false>},
+         {tensor_kernel<32, 2, true>, tensor_kernel<64, 2, true>, tensor_kernel<96, 2, true>, tensor_kernel<128, 2, true>}}};
+    const int many = a.p.Kp > a.p.KC ? 1 : 0, cols = a.p.NC / 32 - 1;
+    auto* kernel = kernels[a.p.nR - 1][many][cols];
+    // the shared-memory limit is raised once per (kernel instance, device)
+    constexpr int kDevices = 64;
+    static std::atomic<size_t> raised[2][2][4][kDevices];
+    std::atomic<size_t>* granted = device >= 0 && device < kDevices ? &raised[a.p.nR - 1][many][cols][device] : nullptr;
+    if (!granted || granted->load(std::memory_order_relaxed) < a.p.smem_bytes) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.p.smem_bytes);
+        if (e != cudaSuccess) return e;
+        if (granted) granted->store(a.p.smem_bytes, std::memory_order_relaxed);
+    }
+    kernel<<<a.p.grid, kThreads, a.p.smem_bytes, stream>>>(a);
+    return cudaGetLastError();
+}
+
+cudaError_t tensor_wait_timeouts(unsigned* count) {
+    unsigned zero = 0;
+    cudaError_t e = cudaMemcpyFromSymbol(count, g_tensor_timeouts, sizeof *count);
+    if (e == cudaSuccess && *count != 0) e = cudaMemcpyToSymbol(g_tensor_timeouts, &zero, sizeof zero);
+    return e;
+}
+
+bool plan_tensor(const PairMap& pm, int H, int W, int sm_count, int max_slices, TensorPlan* out, double* out_us) {
+    if (H < 8 || W < 8 || H > 1024 || W > kTensorMaxRow) return false;
+    const bool shared_rights = pm.n_left == 1 || pm.right_stride == 0;     // every left meets every right
+    double best = 1e30;
+    for (int flip = 0; flip < 2; ++flip) {
+        TensorPlan p{};
+        p.H = H; p.W = W; p.flip = flip;
+        const unsigned m = pm.m, n = pm.n_left;
+        if (shared_rights) {
+            p.groups = 1;
+            p.nA = (int)(flip ? m : n); p.nBt = (int)(flip ? n : m);
+            p.stride_a = (int)(flip ? 1 : m); p.stride_b = (int)(flip ? m : 1);
+        } else {
+            p.groups = n;
+            p.nA = (int)(flip ? m : 1); p.nBt = (int)(flip ? 1 : m);
+            p.stride_a = flip ? 1 : 0; p.stride_b = flip ? 0 : 1;
+            p.group_a = (int)(flip ? m : 1); p.group_b = (int)(flip ? 1 : m); p.group_pairs = (int)m;
+        }
+        if ((long long)p.nA * H > 1 << 30) continue;
+        p.Kp = up(W, 16);
+        for (int NC = 32; NC <= kTensorMaxCols; NC += 32)
+        for (int nB = 1; nB <= std::min(p.nBt, kTensorMaxB); ++nB)
+        for (int nR = 1; nR <= (nB == 1 ? 2 : 1); ++nR)
+        for (int J = 1; J <= std::min(p.nA, kTensorMaxJ); J *= 2)
+        for (int S = 1; S <= std::min(max_slices, H); ++S) {
+            if (S > 1 && (flip || p.nA != 1)) break;
+            if (nB * W > kTensorMaxRow) continue;
+            const int nS = nB * nR;
+            const int dw = 2 * NC / nS / 16 * 16;
+            if (dw < 16) break;
+            p.NC = NC; p.nB = nB; p.nR = nR; p.S = S; p.J = J;
+            p.stack_rows = (p.nA + J - 1) / J * H;
+            p.m_tiles = (unsigned)((p.stack_rows + 128 / J * nR - 1) / (128 / J * nR));
+            p.x_tiles = (2 * W - 1 + dw - 1) / dw;
+            p.DW = up((2 * W - 1 + p.x_tiles - 1) / p.x_tiles, 16);
+            p.b_groups = (unsigned)((p.nBt + nB - 1) / nB);
+            const int rows = (H + S - 1) / S;
+            // a split row: W elements, what the last core matrix reads beyond them, zeros
+            p.row_words = up((W + 14) / 8 * 8 + 8 + 16, 8) / 2;
+            p.res_rows = (128 / J * nR + rows - 1 + nR - 1) / nR;
+            p.AR = nR * p.res_rows * J | 1;
+            // Toeplitz rows of a step, whatever the tile
+            if (((W + 13) / 8 + 1) * nS * 8 > kTensorMaxItems) continue;
+            if (((128 / J * nR + 2 * H + rows) / H + 1) * J > kTensorMaxStack) continue;
+            const auto smem_of = [&] {
+                const size_t a_bytes = std::max<size_t>((size_t)3 * (p.KC / 8) * p.AR * 16, (size_t)kDrainWarps * 16 * (NC + 1) * 4);
+                return a_bytes + (size_t)p.slots * 3 * ((p.DW + p.KC) / 8) * nS * 128 + (size_t)kDrainWarps * J * (NC + 4) * 4 +
+                       (size_t)12 * kRowRing * nB * p.row_words;
+            };
+            bool fits = false;
+            for (p.slots = kTensorMaxSlots; p.slots >= 2; --p.slots) {
+                for (p.KC = std::min(p.Kp, kTensorMaxChunk); p.KC >= (p.slots > 2 ? std::min(p.Kp, 48) : 16); p.KC -= 16)
+                    if (smem_of() <= kSmemLimit - sizeof(Shared) - 1024) { fits = true; break; }
+                if (fits) break;
+            }
+            if (!fits) continue;
+            const int chunks = (p.Kp + p.KC - 1) / p.KC;
+            p.KC = up((p.Kp + chunks - 1) / chunks, 16);
+            // one block per SM: half of tensor memory or more, and the registers, are taken
+            p.smem_bytes = std::max<size_t>(smem_of(), 120 * 1024);
+            if ((double)nB * p.stride_b * (2.0 * H - 1) * (2.0 * W - 1) > 2e9) continue;    // (32-bit column offsets)
+            const unsigned long long grid = (unsigned long long)p.x_tiles * p.groups * p.m_tiles * p.b_groups * S;
+            if (grid > 0x7fffffffull) continue;
+            p.grid = (unsigned)grid;
+            // time of a block in clocks: its matrix products at the tensor cores' rate or that of the
+            // shared memory they read, its drains, its Toeplitz rows; staging once per chunk
+            double sum_clk = 0, max_clk = 0;
+            const int xt_n = std::min(p.x_tiles, 64);
+            for (int xt = 0; xt < xt_n; ++xt) {
+                double clk = 4500.0 + 140.0 * NC;
+                for (int k0 = 0; k0 < p.Kp; k0 += p.KC) {
+                    const int kc = std::min(p.KC, p.Kp - k0);
+                    const int X0 = p.Kp - 1 + W - 1 - xt * p.DW - k0;
+                    double row = 0;
+                    for (int s = 0; s < kc / 16; ++s) {
+                        const int lo = std::max(0, (X0 - W + 1 - 16 * s - 15) & ~7), hi = std::min(p.DW, X0 - 16 * s + 1);
+                        if (hi <= lo) continue;
+                        const double cols = (double)up(hi - lo, 16) * nS;
+                        row += 6 * std::max(cols / 2, 32 + cols / 4) + (row == 0 ? (p.DW * nS - cols) / 2 : 0);
+                    }
+                    if (row == 0) continue;
+                    const int blocks = std::min((W + 13) / 8 + 1, (p.DW + kc) / 8);
+                    const double produce = 440.0 + 210.0 * ((blocks * nS * 8 + kProducers - 1) / kProducers) + 80.0 * ((nB * W + kProducers - 1) / kProducers);
+                    // (a step waits for the slowest of the drain warps: some of them writes a wrapped row in most steps)
+                    const double drain = 110.0 + 3.7 * NC + (J == 1 ? 0.75 : 0.5) * std::min(1.0, 128.0 / J / H) * (300.0 + 9.0 * NC + 4.0 * J * NC);
+                    // (the 128-column build for several chunks spills in its producers)
+                    double c3[3] = {row + 40, p.Kp > p.KC && NC == 128 ? 1.6 * produce : produce, drain};
+                    std::sort(c3, c3 + 3);
+                    clk += (rows + nR - 1) * (c3[2] + 0.5 * c3[1]) + 3.0 * p.AR * (kc / 8) + 1500.0;
+                }
+                sum_clk += clk;
+                max_clk = std::max(max_clk, clk);
+            }
+            const double total = sum_clk * ((double)p.grid / xt_n);
+            const double waves = (double)p.grid / sm_count;
+            // the busiest SM: whole blocks
+            const double clk = p.x_tiles == 1 ? max_clk * (double)(long long)(waves + 0.999999)
+                                              : std::max(max_clk, total / sm_count + 0.5 * max_clk * (waves > 1));
+            double us = clk / 1850.0 + 7.0;
+            if (S > 1) us += 3.0 + (double)S * (2.0 * H - 1) * (2.0 * W - 1) * p.nBt * 4 / 4e6;
+            if (us < best) { best = us; *out = p; }
+        }
+    }
+    *out_us = best;
+    return best < 1e29;
+}
+
+}  // namespace xcorr

@@ -1,0 +1,147 @@
+"""The tensor-core route of the automatic choice (csrc/xcorr_tensor.cu): when it is taken (CPU, from the
+plan text), and its results against the CPU oracle at the edges of its tiles (GPU)."""
+import os
+
+import numpy as np
+import pytest
+
+from conftest import file_to_grouped, grouped_to_file, seeded_inputs
+
+# shapes the planner sends to the tensor cores: one and two Toeplitz rows taken together, one and two
+# matrices interleaved, several matrices B, mirrored results, one to four column chunks, odd sizes, tiles of
+# x shifts, row slices with partial images, groups that fill no tile
+ROUTED = [("n_to_m", 27, 43, 9, 35), ("n_to_m", 32, 32, 32, 64), ("n_to_m", 113, 19, 11, 45), ("n_to_mn", 48, 48, 4, 256),
+          ("n_to_mn", 82, 23, 15, 900), ("one_to_one", 225, 132, 1, 1), ("one_to_one", 256, 256, 1, 1), ("n_to_m", 14, 114, 43, 17),
+          ("one_to_many", 32, 121, 1, 228), ("one_to_many", 64, 64, 1, 129), ("n_to_mn", 41, 50, 3, 333), ("one_to_many", 128, 128, 1, 8)]
+
+
+def plan(xc, shape, hints=None):
+    return xc.describe_plan(*shape, hints)
+
+
+@pytest.mark.parametrize("shape", ROUTED)
+def test_route_and_what_keeps_to_the_tile_kernel(xc, shape):
+    assert plan(xc, shape).startswith("kernel=tensor<")
+    # hints that ask for another plan are obeyed; `reproducible` is met as it is (no atomically added sums)
+    for hints in (dict(kernel="tile"), dict(overlap_rows=1), dict(schedule=1), dict(class_lanes=32), dict(kernel="overlap_wise")):
+        assert "kernel=tensor" not in plan(xc, shape, xc.make_hints(**hints)), hints
+    text = plan(xc, shape)
+    assert "with tile hints kernel=tile" in text
+    # the workspace stays what the tile plan asks for
+    assert xc.workspace_bytes(*shape) == xc.workspace_bytes(*shape, xc.make_hints(kernel="tile"))
+
+
+@pytest.mark.parametrize("shape", [("one_to_one", 16, 16, 1, 1), ("one_to_one", 100, 75, 1, 1), ("n_to_m", 32, 32, 8, 8),
+                                   ("one_to_many", 16, 16, 1, 1000), ("one_to_many", 4, 600, 1, 300), ("n_to_mn", 87, 43, 61, 61)])
+def test_small_calls_and_finer_sums_stay(xc, shape):
+    """Too little work, sizes the route does not take, and plans whose many short sums round less."""
+    assert "kernel=tensor" not in plan(xc, shape)
+
+
+def run(xc, torch, shape, left, right, hints=None, workspace=True):
+    mode, rows, cols, nl, nr = shape
+    guard = 256
+    out_shape = xc.out_shape(mode, rows, cols, nl, nr)
+    n = int(np.prod(out_shape))
+    dl, dr = torch.from_numpy(left).cuda(), torch.from_numpy(right).cuda()
+    whole = torch.full((n + 2 * guard,), -7.25e30, dtype=torch.float32, device="cuda")
+    out = whole[guard:guard + n]
+    out.fill_(float("nan"))
+    wsb = xc.workspace_bytes(mode, rows, cols, nl, nr, hints) if workspace else 0
+    ws = torch.empty(wsb + 16, dtype=torch.uint8, device="cuda")
+    xc.run_device(mode, dl.data_ptr(), dr.data_ptr(), out.data_ptr(), rows, cols, nl, nr, hints,
+                  ws.data_ptr() if wsb else 0, wsb, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert bool((whole[:guard] == -7.25e30).all()) and bool((whole[guard + n:] == -7.25e30).all())
+    return out.reshape(out_shape).cpu().numpy()
+
+
+def reference(oracle, shape, left, right):
+    mode, nl = shape[0], shape[3]
+    threads = os.cpu_count() or 1
+    if mode == "n_to_mn":
+        return file_to_grouped(oracle.run(mode, left, grouped_to_file(right, nl), acc64=True, threads=threads), nl)
+    return oracle.run(mode, left, right, acc64=True, threads=threads)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", ROUTED)
+def test_results_against_the_oracle(xc, oracle, shape):
+    """2-norm within 3.5 units of 2^-24: about one for the rounding towards zero inside tensor memory, 0.2
+    sqrt(row sums) for the sums in registers (at most 1024 / 4 of them here) and a margin; two runs agree bit for bit."""
+    torch = pytest.importorskip("torch")
+    mode, rows, cols, nl, nr = shape
+    left, right = seeded_inputs(rows, cols, nl, nr, 31 * rows + cols)
+    got = run(xc, torch, shape, left, right)
+    assert xc.last_launch().startswith("kernel=tensor<"), xc.last_launch()
+    want = reference(oracle, shape, left, right)
+    assert not np.isnan(got).any()
+    err = np.linalg.norm((got - want).ravel()) / np.linalg.norm(want.ravel())
+    assert err <= 3.5 * 2.0 ** -24, (err * 2 ** 24, xc.last_launch())
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+    assert np.array_equal(got, run(xc, torch, shape, left, right, xc.make_hints(reproducible=1)))
+    xc.check_device()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [("n_to_m", 27, 43, 9, 35), ("n_to_mn", 48, 48, 4, 256), ("one_to_one", 225, 132, 1, 1)])
+@pytest.mark.parametrize("value", [np.nan, np.inf, 1e30, 1e-30])
+def test_operands_outside_the_range_of_the_split(xc, oracle, shape, value):
+    """Infinities and NaN meet exactly the products of the definition (the padding's zeros are not multiplied
+    with them); very large and very small matrices keep their precision."""
+    torch = pytest.importorskip("torch")
+    mode, rows, cols, nl, nr = shape
+    left, right = seeded_inputs(rows, cols, nl, nr, 9)
+    if abs(value) < 1:
+        right[nr // 2] *= np.float32(value)                       # a whole matrix far below the others
+        left[0] *= np.float32(1e8)
+    else:
+        right[nr // 2, rows // 3, cols - 1] = value
+        left[nl - 1, rows - 1, 0] = 0.0                           # inf * 0 where they meet
+    got = run(xc, torch, shape, left, right)
+    assert xc.last_launch().startswith("kernel=tensor<"), xc.last_launch()
+    with np.errstate(all="ignore"):
+        want = reference(oracle, shape, left, right)
+    for g, w in zip(got, want):                                   # per result matrix
+        finite = np.isfinite(w)
+        assert np.array_equal(np.isnan(g), np.isnan(w)) and np.array_equal(g[~finite], w[~finite].astype(np.float32), equal_nan=True)
+        if finite.any():
+            scale = np.abs(w[finite]).max()
+            assert np.abs(g[finite] - w[finite]).max() <= 1e-5 * scale
+
+
+@pytest.mark.gpu
+def test_side_stream_capture_and_missing_workspace(xc, oracle):
+    torch = pytest.importorskip("torch")
+    shape = ("one_to_one", 225, 132, 1, 1)
+    left, right = seeded_inputs(225, 132, 1, 1, 3)
+    want = reference(oracle, shape, left, right)
+    # without the workspace its partial images live in, the call keeps to a plan that needs none
+    got = run(xc, torch, shape, left, right, workspace=False)
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+    # odd addresses: operands and result 4 bytes into a buffer
+    shape = ("n_to_m", 27, 43, 9, 35)
+    left, right = seeded_inputs(27, 43, 9, 35, 4)
+    want = reference(oracle, shape, left, right)
+    n = int(np.prod(xc.out_shape(*shape)))
+    dl = torch.from_numpy(np.concatenate([np.zeros(1, np.float32), left.ravel()])).cuda()
+    dr = torch.from_numpy(np.concatenate([np.zeros(1, np.float32), right.ravel()])).cuda()
+    out = torch.full((n + 1,), float("nan"), dtype=torch.float32, device="cuda")
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+
+    def call(stream):
+        xc.run_device("n_to_m", dl.data_ptr() + 4, dr.data_ptr() + 4, out.data_ptr() + 4, 27, 43, 9, 35, None, 0, 0, stream)
+
+    with torch.cuda.stream(side):
+        call(side.cuda_stream)
+        side.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            call(torch.cuda.current_stream().cuda_stream)
+        out.fill_(float("nan"))
+        graph.replay()
+        side.synchronize()
+    assert xc.last_launch().startswith("kernel=tensor<")
+    got = out[1:].cpu().numpy().reshape(want.shape)
+    assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()

@@ -1,4 +1,5 @@
-// FFT path of the cross-correlation: pad -> batched real-to-complex FFT (cuFFT) -> spectrum
+// FFT path of the cross-correlation, for transforms too large for one SM (the others: xcorr_fft_block.cu) and the
+// raw layout: pad -> batched real-to-complex FFT (cuFFT) -> spectrum
 // product left * conj(right) -> batched complex-to-real FFT (cuFFT) -> unpack.
 //
 // Stands in for the reference's cuFFT algorithms (one_to_one.hpp:888-1170 fft_original_alg_* /
@@ -239,6 +240,11 @@ int fft_run(const float* left, const float* right, float* out, int H, int W, con
         *err = std::string(what) + ": " + cudaGetErrorString(e);
         return true;
     };
+
+    // small enough for one SM: one block per pair does it all
+    cudaError_t block_err = cudaSuccess;
+    if (!raw_result && fft_block_run(left, right, out, H, W, pm, n_right, workspace, lay.total, device, sm_count, stream, &block_err, launches))
+        return cuda_check(block_err, "fft_block_kernel") ? 1 : 0;
 
     // 1. pad both inputs: left matrices first, right matrices after them
     const bool vec = (W % 4 == 0) && reinterpret_cast<uintptr_t>(left) % 16 == 0 &&

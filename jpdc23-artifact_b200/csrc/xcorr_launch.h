@@ -67,6 +67,11 @@ FftLayout fft_workspace_layout(const PairMap& pm, int H, int W, unsigned n_right
 int fft_run(const float* left, const float* right, float* out, int H, int W, const PairMap& pm, unsigned n_right,
             int raw_result, void* workspace, int device, int sm_count, cudaStream_t stream, std::string* err,
             int* launches);
+// The normalized layout in one block per pair, for sizes whose half spectrum fits one SM (xcorr_fft_block.cu).
+// false: not such a size (nothing was launched); true: *err is the launches' status.
+bool fft_block_run(const float* left, const float* right, float* out, int H, int W, const PairMap& pm, unsigned n_right,
+                   void* workspace, size_t workspace_bytes, int device, int sm_count, cudaStream_t stream, cudaError_t* err,
+                   int* launches);
 void fft_release_plans();
 
 }  // namespace xcorr

@@ -14,7 +14,7 @@
 // Twiddles come from tables computed once per block (sincospif).
 // Bound by shared-memory traffic, 16 bytes a point and pass, and the latency of a pass between two barriers; the
 // result is written once, the inputs read once.  Measured on B200 against pad, cuFFT, product, cuFFT, unpack (us):
-// 64 x 64 1 x 512 106 -> 62, 90 x 75 4 x 48 55 -> 35, 60 x 60 1 x 1500 285 -> 145, one 30 x 30 pair 33 -> 17.
+// 64 x 64 1 x 512 106 -> 60, 90 x 75 4 x 48 55 -> 35, 60 x 60 1 x 1500 285 -> 141, one 60 x 60 pair 33 -> 26.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <atomic>
@@ -444,7 +444,11 @@ bool fft_block_run(const float* left, const float* right, float* out, int H, int
     float2* store = static_cast<float2*>(workspace);
     const auto run = [&](bool pair, unsigned grid) -> cudaError_t {
         ++*launches;
-        // three blocks of 256 threads per SM where they fit, two of 384, else one of 512
+        // three blocks of 256 threads per SM where they fit, two of 384, else one of 512; no more blocks than SMs:
+        // 512 threads, the time is one block's (one 60 x 60 pair 29 -> 26 us, 64 x 64 9 x 14 43 -> 27 us with the
+        // launch saved below; the left spectra of 64 x 64 1 x 512, one block before all others, 62 -> 60 us)
+        if (grid <= (unsigned)sm_count && bytes > 12 * 1024)
+            return pair ? launch<512, 1, true>(a, grid, bytes, device, stream) : launch<512, 1, false>(a, grid, bytes, device, stream);
         if (bytes <= 75 * 1024)
             return pair ? launch<256, 3, true>(a, grid, bytes, device, stream) : launch<256, 3, false>(a, grid, bytes, device, stream);
         if (bytes <= 113 * 1024)

@@ -30,8 +30,8 @@
 // Tried and left: writing a wrapped row from its lane's registers straight to global memory (one 4-byte store in
 // flight per SM every 7 clocks: 64 x 64 1 x 512 took 327 us), 4 and 16 matrices interleaved (fewer wraps, but all
 // warps wait for the one that writes: 32 x 32 32 x 64 88 us against 70).
-// Measured on B200 (us, tile kernel -> this one): 256 x 256 one pair 168 -> 95, 64 x 64 1 x 512 353 -> 119,
-// 32 x 32 32 x 64 101 -> 68, 48 x 48 16 x 2048 450 -> 201, 27 x 43 9 x 35 53 -> 34.
+// Measured on B200 (us, tile kernel -> this one): 256 x 256 one pair 168 -> 94, 64 x 64 1 x 512 353 -> 121,
+// 32 x 32 32 x 64 101 -> 69, 48 x 48 16 x 2048 450 -> 205, 27 x 43 9 x 35 53 -> 33, 256 x 256 1 x 32 4657 -> 1609.
 //
 // Roles of a block (12 warps): warps 0..7 drain tensor memory into register sums and write results,
 // 8..10 build the Toeplitz rows, warp 11 issues the matrix products.
@@ -101,14 +101,23 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
 }
+// KEEP: what becomes of the A operand in the tensor core's collector buffer -- read and kept for the next
+// product (fill), taken from there for the last time (lastuse), or neither.
+enum Keep { kDiscard, kFill, kLastUse };
+#define XC_MMA(OP) \
+    asm volatile("{ .reg .pred p; .reg .b64 a, b;\n\t" \
+                 "mov.b64 a, {%1, %3};\n\t" \
+                 "mov.b64 b, {%2, %3};\n\t" \
+                 "setp.ne.b32 p, %5, 0;\n\t" \
+                 "tcgen05.mma.cta_group::1.kind::f16.collector::a::" OP " [%0], a, b, %4, p; }" \
+                 :: "r"(d), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory")
+template<Keep KEEP = kDiscard>
 __device__ __forceinline__ void tc_mma(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{ .reg .pred p; .reg .b64 a, b;\n\t"
-                 "mov.b64 a, {%1, %3};\n\t"
-                 "mov.b64 b, {%2, %3};\n\t"
-                 "setp.ne.b32 p, %5, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p; }"
-                 :: "r"(d), "r"(a_lo), "r"(b_lo), "r"(desc_hi), "r"(idesc), "r"(accumulate) : "memory");
+    if (KEEP == kFill) XC_MMA("fill");
+    else if (KEEP == kLastUse) XC_MMA("lastuse");
+    else XC_MMA("discard");
 }
+#undef XC_MMA
 // Asynchronous: the registers are the caller's after tc_load_wait.
 __device__ __forceinline__ void tc_load(uint32_t addr, uint32_t (&r)[16]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -605,10 +614,12 @@ __global__ void __launch_bounds__(kThreads, 1) tensor_kernel(const __grid_consta
                         if (s >= n_steps) break;
                         const uint32_t a = a0 + st[s].a_off, b = b0 + st[s].b_off, d = d0 + st[s].d_off, id = st[s].idesc;
                         if (s > 0) tc_mma(d, a + 2 * a_part16, b, desc_hi, id, 1);
-                        tc_mma(d, a, b + 2 * bp, desc_hi, id, 1);
-                        tc_mma(d, a + a_part16, b + bp, desc_hi, id, 1);
-                        tc_mma(d, a + a_part16, b, desc_hi, id, 1);
-                        tc_mma(d, a, b + bp, desc_hi, id, 1);
+                        // (the middle and the high part of A are each read once for two products: 27 x 43 9 x 35 34.7 ->
+                        // 32.8 us, one 256 x 256 pair 95.8 -> 94.2; nothing where the wrapped rows set the pace)
+                        tc_mma<kFill>(d, a + a_part16, b + bp, desc_hi, id, 1);
+                        tc_mma<kLastUse>(d, a + a_part16, b, desc_hi, id, 1);
+                        tc_mma<kFill>(d, a, b + 2 * bp, desc_hi, id, 1);
+                        tc_mma<kLastUse>(d, a, b + bp, desc_hi, id, 1);
                     }
 #pragma unroll
                     for (int s = 0; s < kMaxSteps; ++s) {

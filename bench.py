@@ -368,10 +368,18 @@ def reference_gpu_baseline(dev, launch, iters=20, launch_on=None):
     return out
 
 
+def fft_figures(k, ms, hbm_peak):
+    """What one call of the FFT path of `ms` milliseconds amounts to.  `bytes`: every input read and every
+    result written once, whatever its kernels move."""
+    moved = bytes_of(k)
+    return {"ms": ms, "equivalent_gflops": flop_of(k) / (ms * 1e-3) / 1e9, "bytes": moved,
+            "hbm_gbs": moved / (ms * 1e-3) / 1e9, "frac_hbm_measured": moved / (ms * 1e-3) / 1e9 / hbm_peak}
+
+
 def fft_path_timings(xc, dev, stream, hbm_peak, iters=20):
     """The FFT path (xcorr_fft_f32, normalized layout) on the same resident inputs: the
     algorithmic alternative the reference carries next to the direct kernels.  Reported beside
-    the headline, not part of it.  `bytes`: every input read and every result written once."""
+    the headline, not part of it."""
     import torch
     out = {}
     for k, (mode, r, c, nl, nr) in CONFIGS.items():
@@ -395,70 +403,8 @@ def fft_path_timings(xc, dev, stream, hbm_peak, iters=20):
         b.record()
         torch.cuda.synchronize()
         ms = a.elapsed_time(b) / iters
-        pairs = pairs_of(mode, nl, nr)
-        traffic = 4 * ((nl + nr) * r * c + pairs * (2 * r - 1) * (2 * c - 1))
-        diff = float((res - d["out"]).abs().max() / res.abs().max())
-        # this library's call timed the same way: `iters` back-to-back calls between two events
-        for _ in range(3):
-            launch(k)
-        torch.cuda.synchronize()
-        a.record()
-        for _ in range(iters):
-            launch(k)
-        b.record()
-        torch.cuda.synchronize()
-        ours = a.elapsed_time(b) / iters
-        out["per_config"][k] = {"ms": ms, "gflops": flop_of(k) / (ms * 1e-3) / 1e9,
-                                "max_abs_diff_to_ours_over_max": diff, "ours_ms": ours, "speedup": ms / ours}
-        if mode == "one_to_one" and wps is not None and r * c <= 32 * 32 and launch_on is not None:
-            # a few microseconds each: back-to-back calls above time the host; these are graph replays
-            ref_us = wps.graph_us(L, R, O, r, c, 16)
-            ours_us = graph_replay_us(lambda s_: launch_on(k, s_))
-            out["per_config"][k].update({"device_us": ref_us, "ours_device_us": ours_us,
-                                         "device_speedup": ref_us / ours_us if ref_us > 0 else None,
-                                         "device_timing": "20 launches in a CUDA graph, 10 replays between two events"})
-    return out
-
-
-def fft_path_timings(xc, dev, stream, hbm_peak, iters=20):
-    """The FFT path (xcorr_fft_f32, normalized layout) on the same resident inputs: the
-    algorithmic alternative the reference carries next to the direct kernels.  Reported beside
-    the headline, not part of it.  `bytes`: every input read and every result written once."""
-    import torch
-    out = {}
-    for k, (mode, r, c, nl, nr) in CONFIGS.items():
-        d = dev[k]
-        wsb = xc.fft_workspace_bytes(mode, r, c, nl, nr)
-        ws = torch.empty(wsb + 256, dtype=torch.uint8, device="cuda")
-        base = (ws.data_ptr() + 255) // 256 * 256
-        res = torch.empty_like(d["out"])
-
-        def run():
-            xc.run_fft_device(mode, d["left"].data_ptr(), d["right"].data_ptr(), res.data_ptr(), r, c, nl, nr,
-                              "normalized", base, wsb, stream)
-        for _ in range(3):
-            run()
-        a = torch.cuda.Event(enable_timing=True)
-        b = torch.cuda.Event(enable_timing=True)
-        torch.cuda.synchronize()
-        a.record()
-        for _ in range(iters):
-            run()
-        b.record()
-        torch.cuda.synchronize()
-        ms = a.elapsed_time(b) / iters
-        pairs = pairs_of(mode, nl, nr)
-        real, cplx = 4 * r * c * 4, 2 * r * (c + 1) * 8          # bytes of one padded matrix / one spectrum
-        n_in = nl + nr
-        traffic = (n_in * (r * c * 4 + real)                      # pad
-                   + n_in * (real + cplx)                         # forward
-                   + pairs * 3 * cplx                             # product (left spectra re-read from L2)
-                   + pairs * (cplx + real)                        # inverse
-                   + pairs * (real + (2 * r - 1) * (2 * c - 1) * 4))   # unpack
         diff = float((res - d["out"]).abs().max() / d["out"].abs().max())
-        out[k] = {"ms": ms, "equivalent_gflops": flop_of(k) / (ms * 1e-3) / 1e9, "bytes": traffic,
-                  "hbm_gbs": traffic / (ms * 1e-3) / 1e9, "frac_hbm_measured": traffic / (ms * 1e-3) / 1e9 / hbm_peak,
-                  "max_abs_diff_to_direct_over_max": diff}
+        out[k] = dict(fft_figures(k, ms, hbm_peak), max_abs_diff_to_direct_over_max=diff)
         del ws, res
     return out
 

@@ -67,6 +67,46 @@ def test_two_gloo_ranks_split_every_configuration_without_gaps(xc):
         assert abs(parts[0][1] - parts[1][1]) <= 1
 
 
+def test_functions_are_defined_once_and_name_nothing_undefined():
+    """A second definition hides the first, and a name that exists nowhere is found only when it runs."""
+    import ast
+    import builtins
+    import collections
+    tree = ast.parse(open(os.path.join(ROOT, "bench.py")).read())
+    defined = [n.name for n in tree.body if isinstance(n, (ast.FunctionDef, ast.ClassDef))]
+    assert [n for n, c in collections.Counter(defined).items() if c > 1] == []
+    module = {t.id for n in tree.body for t in ast.walk(n) if isinstance(t, ast.Name) and not isinstance(t.ctx, ast.Load)
+              and not isinstance(n, (ast.FunctionDef, ast.ClassDef))} | set(defined) | set(dir(builtins)) | {"__file__"}
+    module |= {a.asname or a.name.split(".")[0] for n in tree.body if isinstance(n, (ast.Import, ast.ImportFrom)) for a in n.names}
+    for f in tree.body:
+        if not isinstance(f, ast.FunctionDef):
+            continue
+        local = set(module)
+        for n in ast.walk(f):
+            if isinstance(n, ast.Name) and not isinstance(n.ctx, ast.Load):
+                local.add(n.id)
+            elif isinstance(n, ast.arg):
+                local.add(n.arg)
+            elif isinstance(n, (ast.FunctionDef, ast.ClassDef)):
+                local.add(n.name)
+            elif isinstance(n, (ast.Import, ast.ImportFrom)):
+                local |= {a.asname or a.name.split(".")[0] for a in n.names}
+            elif isinstance(n, ast.ExceptHandler) and n.name:
+                local.add(n.name)
+        missing = {n.id for n in ast.walk(f) if isinstance(n, ast.Name) and n.id not in local}
+        assert not missing, (f.name, missing)
+
+
+def test_fft_path_reports_the_compulsory_bytes():
+    """`bytes` of the FFT path are those its text states -- inputs read once, results written once -- so that a
+    fraction of the memory bandwidth cannot be claimed for passes that are not made."""
+    sys.path.insert(0, ROOT)
+    import bench
+    f = bench.fft_figures("C3", 0.1, 6500.0)
+    assert f["bytes"] == 4 * (513 * 64 * 64 + 512 * 127 * 127)
+    assert abs(f["hbm_gbs"] - f["bytes"] / 1e-4 / 1e9) < 1e-6 and abs(f["frac_hbm_measured"] - f["hbm_gbs"] / 6500.0) < 1e-12
+
+
 def test_reference_arm_prints_one_line_from_rank_zero():
     """`bench.py --impl reference` under a two-rank launch: rank 0 alone times the reference's
     CPU code and prints the line; the other rank exits without work."""

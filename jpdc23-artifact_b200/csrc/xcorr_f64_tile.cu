@@ -25,7 +25,6 @@
 // would not fit; the slices' sums are then added with red.global.add.f64 onto the zeroed output.
 #include <cuda_runtime.h>
 #include <algorithm>
-#include <atomic>
 #include <cstdio>
 #include <cstdint>
 #include <cstdlib>
@@ -34,6 +33,7 @@
 #include <cstdint>
 
 #include "xcorr_launch.h"
+#include "xcorr_smem.h"
 
 namespace xcorr {
 namespace {
@@ -313,14 +313,11 @@ bool plan_tile_f64(const PairMap& pm, int H, int W, int sm_count, size_t smem_li
 }
 
 cudaError_t launch_tile_f64(const TileArgs64& a, int device, cudaStream_t stream) {
-    constexpr int kDevices = 64;
-    static std::atomic<size_t> raised[kDevices];
-    if (a.p.smem_bytes > 48 * 1024 &&
-        !(device >= 0 && device < kDevices && raised[device].load(std::memory_order_relaxed) >= a.p.smem_bytes)) {
-        cudaError_t e = cudaFuncSetAttribute(tile_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.p.smem_bytes);
-        if (e != cudaSuccess) return e;
-        if (device >= 0 && device < kDevices) raised[device].store(a.p.smem_bytes, std::memory_order_relaxed);
-    }
+    static SmemLimit limit;
+    const cudaError_t e = limit.allow(device, a.p.smem_bytes, [](size_t bytes) {
+        return cudaFuncSetAttribute(tile_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    });
+    if (e != cudaSuccess) return e;
     tile_f64_kernel<<<a.p.grid, a.p.threads, a.p.smem_bytes, stream>>>(a);
     return cudaGetLastError();
 }

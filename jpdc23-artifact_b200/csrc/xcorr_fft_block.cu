@@ -17,10 +17,10 @@
 // 64 x 64 1 x 512 106 -> 60, 90 x 75 4 x 48 55 -> 35, 60 x 60 1 x 1500 285 -> 141, one 60 x 60 pair 33 -> 26.
 #include <cuda_runtime.h>
 #include <algorithm>
-#include <atomic>
 #include <cstdint>
 
 #include "xcorr_launch.h"
+#include "xcorr_smem.h"
 
 namespace xcorr {
 
@@ -393,14 +393,11 @@ size_t smem_bytes(const Dim& rows, const Dim& cols) {
 
 template<int THREADS, int BLOCKS, bool PAIR>
 cudaError_t launch(const FftBlockArgs& a, unsigned grid, size_t bytes, int device, cudaStream_t stream) {
-    constexpr int kDevices = 64;
-    static std::atomic<size_t> raised[kDevices];
-    std::atomic<size_t>* granted = device >= 0 && device < kDevices ? &raised[device] : nullptr;
-    if (bytes > 48 * 1024 && (!granted || granted->load(std::memory_order_relaxed) < bytes)) {
-        const cudaError_t e = cudaFuncSetAttribute(fft_block_kernel<THREADS, BLOCKS, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e != cudaSuccess) return e;
-        if (granted) granted->store(bytes, std::memory_order_relaxed);
-    }
+    static SmemLimit limit;
+    const cudaError_t e = limit.allow(device, bytes, [](size_t size) {
+        return cudaFuncSetAttribute(fft_block_kernel<THREADS, BLOCKS, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)size);
+    });
+    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t config{};
     config.gridDim = dim3(grid);
     config.blockDim = dim3(THREADS);

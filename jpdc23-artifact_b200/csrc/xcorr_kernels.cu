@@ -12,12 +12,12 @@
 //   warp_per_overlap_kernel one warp per overlap (naive_warp_per_shift.cu:192-244).
 // plus the fixed-order reduction of workspace partials and the FFMA peak probe.
 #include <cuda_runtime.h>
-#include <atomic>
 #include <cstdint>
 #include <mutex>
 
 #include "xcorr_plan.h"
 #include "xcorr_launch.h"
+#include "xcorr_smem.h"
 
 namespace xcorr {
 
@@ -1336,22 +1336,17 @@ __global__ void __launch_bounds__(1024) ffma_probe_kernel(float* sink, float b, 
 // ------------------------------------------------------------------------------------------
 // launchers
 // ------------------------------------------------------------------------------------------
-// Kernels that need more than 48 KB of dynamic shared memory have the limit raised once per
-// (kernel instance, device); `raised` remembers the largest size granted so far.
-constexpr int kAttrDevices = 64;
 template<typename K>
-static cudaError_t allow_smem(K kernel, std::atomic<size_t>* raised, int device, size_t bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
-    if (device >= 0 && device < kAttrDevices && raised[device].load(std::memory_order_relaxed) >= bytes) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess && device >= 0 && device < kAttrDevices) raised[device].store(bytes, std::memory_order_relaxed);
-    return e;
+static cudaError_t allow_smem(K kernel, SmemLimit& limit, int device, size_t bytes) {
+    return limit.allow(device, bytes, [&](size_t size) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)size);
+    });
 }
 
 template<int TY, int BOUND, int VARIANT>
 static cudaError_t launch_tile_instance(const TileArgs& a, int device, cudaStream_t stream) {
-    static std::atomic<size_t> raised[kAttrDevices];
-    cudaError_t e = allow_smem(tile_kernel<TY, BOUND, VARIANT>, raised, device, a.p.smem_bytes);
+    static SmemLimit limit;
+    cudaError_t e = allow_smem(tile_kernel<TY, BOUND, VARIANT>, limit, device, a.p.smem_bytes);
     if (e != cudaSuccess) return e;
     tile_kernel<TY, BOUND, VARIANT><<<a.p.grid, a.p.threads, a.p.smem_bytes, stream>>>(a);
     return cudaGetLastError();
@@ -1457,8 +1452,8 @@ size_t staged_smem_bytes(const StagedArgs& a) {
 
 template<int RMAX>
 static cudaError_t launch_staged_instance(const StagedArgs& a, dim3 grid, size_t smem, int device, cudaStream_t stream) {
-    static std::atomic<size_t> raised[kAttrDevices];
-    cudaError_t e = allow_smem(warp_staged_kernel<RMAX>, raised, device, smem);
+    static SmemLimit limit;
+    cudaError_t e = allow_smem(warp_staged_kernel<RMAX>, limit, device, smem);
     if (e != cudaSuccess) return e;
     warp_staged_kernel<RMAX><<<grid, a.shifts * 32, smem, stream>>>(a);
     return cudaGetLastError();

@@ -38,12 +38,12 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <algorithm>
-#include <atomic>
 #include <climits>
 #include <cstdint>
 
 #include "xcorr_plan.h"
 #include "xcorr_launch.h"
+#include "xcorr_smem.h"
 
 namespace xcorr {
 
@@ -731,15 +731,11 @@ cudaError_t launch_tensor(const TensorArgs& a, int device, cudaStream_t stream) 
          {tensor_kernel<32, 2, true>, tensor_kernel<64, 2, true>, tensor_kernel<96, 2, true>, tensor_kernel<128, 2, true>}}};
     const int many = a.p.Kp > a.p.KC ? 1 : 0, cols = a.p.NC / 32 - 1;
     auto* kernel = kernels[a.p.nR - 1][many][cols];
-    // the shared-memory limit is raised once per (kernel instance, device)
-    constexpr int kDevices = 64;
-    static std::atomic<size_t> raised[2][2][4][kDevices];
-    std::atomic<size_t>* granted = device >= 0 && device < kDevices ? &raised[a.p.nR - 1][many][cols][device] : nullptr;
-    if (!granted || granted->load(std::memory_order_relaxed) < a.p.smem_bytes) {
-        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)a.p.smem_bytes);
-        if (e != cudaSuccess) return e;
-        if (granted) granted->store(a.p.smem_bytes, std::memory_order_relaxed);
-    }
+    static SmemLimit limits[2][2][4];
+    const cudaError_t e = limits[a.p.nR - 1][many][cols].allow(device, a.p.smem_bytes, [&](size_t bytes) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    });
+    if (e != cudaSuccess) return e;
     kernel<<<a.p.grid, kThreads, a.p.smem_bytes, stream>>>(a);
     return cudaGetLastError();
 }

@@ -1373,7 +1373,7 @@ int32_t xcorr_describe_plan(int32_t mode, uint32_t rows, uint32_t cols, uint32_t
             text = describe_plan(p);
             TensorPlan tp{};
             if (tensor_auto(hints, pm, (int)rows, (int)cols, dev, p, p.combine == kWorkspace ? p.S : 1, &tp))
-                text = describe_plan(tp) + "; with tile hints " + text;
+                text = describe_plan(tp);
         }
     } else {
         return fail(XCORR_ERR_INVALID_HINT, "unknown kernel family");

@@ -251,11 +251,15 @@ def config_inputs(k):
     return mode, left, right
 
 
+@pytest.mark.parametrize("kernel,route", [("auto", None), ("tile", "kernel=tile<")])
 @pytest.mark.parametrize("k", sorted(CONFIGS))
-def test_benchmark_configs_full_size_against_oracle(xc, oracle, k):
+def test_benchmark_configs_full_size_against_oracle(xc, oracle, k, kernel, route):
     mode, left, right = config_inputs(k)
     want = oracle_grouped(oracle, mode, left, right, acc64=True)
-    got = gpu_run(xc, mode, left, right)
+    got = gpu_run(xc, mode, left, right, xc.make_hints(kernel=kernel))
+    # the automatic choice: one warp per overlap for the single small pair, the tensor cores for the others
+    route = route or ("kernel=warp_per_overlap" if k == "C1" else "kernel=tensor<")
+    assert xc.last_launch().startswith(route), xc.last_launch()
     assert not np.isnan(got).any(), xc.last_launch()
     err = rel_err(got, want)
     assert err <= REL_TOL, (k, err, xc.last_launch())

@@ -25,8 +25,8 @@ def test_route_and_what_keeps_to_the_tile_kernel(xc, shape):
     # hints that ask for another plan are obeyed; `reproducible` is met as it is (no atomically added sums)
     for hints in (dict(kernel="tile"), dict(overlap_rows=1), dict(schedule=1), dict(class_lanes=32), dict(kernel="overlap_wise")):
         assert "kernel=tensor" not in plan(xc, shape, xc.make_hints(**hints)), hints
-    text = plan(xc, shape)
-    assert "with tile hints kernel=tile" in text
+    # one plan, the one that runs
+    assert plan(xc, shape).count("kernel=") == 1 and plan(xc, shape).endswith("}")
     # the workspace stays what the tile plan asks for
     assert xc.workspace_bytes(*shape) == xc.workspace_bytes(*shape, xc.make_hints(kernel="tile"))
 
@@ -74,6 +74,7 @@ def test_results_against_the_oracle(xc, oracle, shape):
     left, right = seeded_inputs(rows, cols, nl, nr, 31 * rows + cols)
     got = run(xc, torch, shape, left, right)
     assert xc.last_launch().startswith("kernel=tensor<"), xc.last_launch()
+    assert xc.last_launch() == plan(xc, shape)
     want = reference(oracle, shape, left, right)
     assert not np.isnan(got).any()
     err = np.linalg.norm((got - want).ravel()) / np.linalg.norm(want.ravel())

@@ -641,26 +641,34 @@ bool tiny_auto(const xcorr_hints* h, const PairMap& pm, uint32_t rows, uint32_t 
 }
 
 // Whether the automatic choice runs this call on the tensor cores: no hint asks for a plan of another
-// kernel and their estimate beats the tile plan's by a margin.
+// kernel, no plan less precise than the tile kernel's is
+// considered, and the estimate beats the tile plan's by a margin.
 bool tensor_auto(const xcorr_hints* h, const PairMap& pm, int H, int W, const DeviceInfo& dev, const TilePlan& tile,
                  int max_slices, TensorPlan* out) {
     if (h && (h->kernel != XCORR_KERNEL_AUTO || h->combine || h->overlap_rows || h->class_lanes || h->warps_x ||
               h->warps_y || h->row_slices || h->schedule || h->block_threads || h->fused_rows))
         return false;
     if (dev.smem_optin < (size_t)kSmemLimit) return false;
+    // No less precise than the tile plan, whose sum of n products taken one after the other is off by 0.185 sqrt(n) units
+    // of 2^-24 of the result, and by less where it happens to be taken in parts (fitted to 90 measured plans, uniform
+    // operands; 64 x 64 in one: 11.8).
+    const double parts = tile.schedule == kSchedStreamK ? std::max(1.0, (double)tile.grid / tile.tasks)
+                       : tile.schedule == kSchedStatic ? (double)tile.S : 1.0;
+    const double max_err2 = 0.0342 * ((double)H * W / (parts * parts) + parts);
     struct Key {
         uint32_t n_left, m, right_stride;
         int H, W, sm_count, max_slices;
+        double max_err2;
         bool operator==(const Key& o) const {
             return n_left == o.n_left && m == o.m && right_stride == o.right_stride && H == o.H && W == o.W &&
-                   sm_count == o.sm_count && max_slices == o.max_slices;
+                   sm_count == o.sm_count && max_slices == o.max_slices && max_err2 == o.max_err2;
         }
     };
     struct Entry { Key key; TensorPlan plan; double est_us; };
     static std::mutex mutex;                       // plans are remembered like the tile kernel's
     static Entry cache[kPlanCacheSize];
     static int used = 0, next = 0;
-    const Key k{pm.n_left, pm.m, pm.right_stride, H, W, dev.sm_count, max_slices};
+    const Key k{pm.n_left, pm.m, pm.right_stride, H, W, dev.sm_count, max_slices, max_err2};
     Entry e{};
     bool found = false;
     {
@@ -670,22 +678,11 @@ bool tensor_auto(const xcorr_hints* h, const PairMap& pm, int H, int W, const De
     }
     if (!found) {
         e.key = k;
-        if (!plan_tensor(pm, H, W, dev.sm_count, max_slices, &e.plan, &e.est_us)) e.est_us = 1e30;
+        if (!plan_tensor(pm, H, W, dev.sm_count, max_slices, max_err2, &e.plan, &e.est_us)) e.est_us = 1e30;
         std::lock_guard<std::mutex> lock(mutex);
         cache[used < kPlanCacheSize ? used++ : next++ % kPlanCacheSize] = e;
     }
     if (!(e.est_us < 0.85 * tile.est_us)) return false;
-    // No less precise than the tile plan.  Error in units of 2^-24 of the result, fitted to 90 measured plans
-    // (uniform operands): a sum of n products taken one after the other is off by 0.185 sqrt(n), and by less
-    // where a plan happens to take it in parts; the tensor cores lose about one unit to rounding towards zero
-    // and 0.2 sqrt(n) to the sums of the rows (87 x 43 61 x 61, cut into 43 parts or more: 1.8 against 2.2;
-    // 64 x 64 1 x 512, in one: 11.8 against 2.0).
-    const double parts = tile.schedule == kSchedStreamK ? std::max(1.0, (double)tile.grid / tile.tasks)
-                       : tile.schedule == kSchedStatic ? (double)tile.S : 1.0;
-    const double sums = (double)H * ((e.plan.Kp + e.plan.KC - 1) / e.plan.KC);
-    const double tile_err2 = 0.0342 * ((double)H * W / (parts * parts) + parts);
-    const double tensor_err2 = 1.0 + 0.04 * (sums / ((double)e.plan.S * e.plan.S) + e.plan.S);
-    if (tensor_err2 > tile_err2) return false;
     *out = e.plan;
     return true;
 }
@@ -751,7 +748,7 @@ std::string describe_plan(const TensorPlan& p) {
     std::snprintf(buf, sizeof buf,
                   "kernel=tensor<%d> grid=(%u,1,1) block=(%d,1,1) smem=%zu tensor{H=%d W=%d side=%s matrices=%d rows=%d interleave=%d x_tiles=%d "
                   "x_shifts=%d chunk=%d slots=%d S=%d combine=%s}",
-                  p.NC, p.grid, kTensorThreads, p.smem_bytes, p.H, p.W, p.flip ? "right" : "left", p.nB, p.nR, p.J, p.x_tiles, p.DW,
+                  p.D, p.grid, tensor_threads(p.D), p.smem_bytes, p.H, p.W, p.flip ? "right" : "left", p.nB, p.nR, p.J, p.x_tiles, p.DW,
                   p.KC, p.slots, p.S, p.S > 1 ? "workspace" : "store");
     return buf;
 }

@@ -11,8 +11,9 @@ cudaError_t launch_tile(const TileArgs& a, int device, cudaStream_t stream);
 cudaError_t launch_reduce_partials(const float* ws, float* out, unsigned long long total_out,
                                    int H, int W, int Hp, int S, int sm_count, cudaStream_t stream);
 // Tensor cores (xcorr_tensor.cu).  plan_tensor returns false where no plan fits; max_slices > 1 allows
-// row slices with partial images (one matrix on the A side).  *est_us is its estimate of the call.
-bool plan_tensor(const PairMap& pm, int H, int W, int sm_count, int max_slices, TensorPlan* out, double* est_us);
+// row slices with partial images (one matrix on the A side); max_err2 bounds the squared 2-norm error it is estimated to
+// have, in units of 2^-24 of the result (uniform operands).  *est_us is its estimate of the call.
+bool plan_tensor(const PairMap& pm, int H, int W, int sm_count, int max_slices, double max_err2, TensorPlan* out, double* est_us);
 cudaError_t launch_tensor(const TensorArgs& a, int device, cudaStream_t stream);
 cudaError_t tensor_wait_timeouts(unsigned* count);   // as tile_stage_timeouts
 cudaError_t launch_overlap_wise(const float* left, const float* right, float* out, int H, int W,

@@ -125,17 +125,20 @@ struct TileArgs64 {
 };
 
 // Plan and arguments of the tensor-core kernel (xcorr_tensor.cu).
-constexpr int kTensorThreads = 384;
 constexpr int kTensorMaxChunk = 64;   // columns of the A side staged at once, and summed in tensor memory
 constexpr int kTensorMaxSlots = 4;    // Toeplitz rows in flight
 constexpr int kTensorMaxB = 12;       // B matrices of a block
 constexpr int kTensorMaxRow = 576;    // elements of one row of a block's B matrices
 constexpr int kTensorMaxItems = 576;  // 8-element rows of the core matrices of a step
-constexpr int kTensorMaxCols = 128;   // result columns of a drain warp
+constexpr int kTensorMaxCols = 256;   // result columns of a block
 constexpr int kTensorMaxJ = 2;        // A matrices interleaved row by row
 constexpr int kTensorMaxStack = 64;   // A matrices a block's rows can touch
 // instruction descriptor without its N: 32-bit accumulators, bfloat16 operands, both K-major, M = 128
 constexpr uint32_t kTensorIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);
+// drain warps for 32 rows and 32 columns each (256 columns: 64), three producer warps and one that issues the products
+template<int COLS> constexpr int kTensorDrainWarps = COLS == 64 ? 8 : 16;
+template<int COLS> constexpr int kTensorThreads = 32 * (kTensorDrainWarps<COLS> + 4);
+inline int tensor_threads(int cols) { return cols == 64 ? kTensorThreads<64> : cols == 128 ? kTensorThreads<128> : kTensorThreads<256>; }
 struct TensorPlan {
     int H, W;
     int flip;          // 0: A side = left matrices; 1: A side = right matrices (results written mirrored)
@@ -150,7 +153,7 @@ struct TensorPlan {
     int DW;            // x shifts of a tile, a multiple of 16
     int nB;            // B matrices of a block
     int nR;            // rows of a B matrix taken together (1 or 2)
-    int NC;            // result columns per drain warp: DW * nB * nR <= 2 * NC
+    int D;             // result columns of a block, 64, 128 or 256: DW * nB * nR <= D
     int Kp, KC;        // padded columns, columns staged at once (multiples of 16)
     int AR;            // staged rows of the A side (an odd number)
     int res_rows;      // staged stack rows of one residue mod nR

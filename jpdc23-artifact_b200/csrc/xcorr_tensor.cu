@@ -1,11 +1,19 @@
 // Direct cross-correlation on the tensor cores (tcgen05, sm_100a), at single precision.
 //
-// A float is the exact sum of three bfloat16 values, x = h + m + l (8 bits of the significand each),
-// so a product of two floats is nine bfloat16 products; the six that reach 2^-18 of it (hh, hm, mh,
-// hl, mm, lh) are taken and the three below 2^-26 are not.  Bfloat16 products are exact in the
-// tensor cores' 32-bit accumulators.  Those accumulators round towards zero, so no sum stays in them
-// for long: one right row (at most kTensorMaxChunk columns of it) is summed in tensor memory, small
-// products first, and then added to sums in registers, rounded to nearest.
+// A float is the exact sum of three bfloat16 values, x = h + m + l (8 bits of the significand each; elements from
+// 2^-110 up), so a product of two floats is nine bfloat16 products, exact in the tensor cores' 32-bit accumulators.
+// Six are taken.  Of the three left out, ml and lm can reach 2^-25 of the product each and ll 2^-34 (h and m are
+// rounded to nearest: m is up to 2^-8 of x, l up to 2^-17); with ml and lm taken too no error measured changes.
+// The accumulators round towards zero.  So the large products (hh: 16 bits, their sum of one row mostly exact) are
+// summed apart from the small ones, whose rounding is 2^-8 of theirs, and both only over one right row (at most
+// kTensorMaxChunk columns of it): row sums are added to nearest in registers, large and small apart, and the two sums
+// meet once, when a result is written.  (All six in one accumulator: every result 0.6 to 1.2 units of 2^-24 too
+// small, overlaps of up to 15 products and sparse operands off by up to twice what FFMAs lose.)  2-norm error against
+// double in units of 2^-24, tile kernel -> this one: uniform operands 64 x 64 11.8 -> 2.0, 48 x 48 8.8 -> 1.7, 32 x 32
+// 5.9 -> 1.4, 27 x 43 6.2 -> 1.4, one 256 x 256 pair 2.3 -> 1.5; normal 12.8 -> 2.2, 9.6 -> 1.9, 6.4 -> 1.6, 6.9 -> 1.5,
+// 10.4 -> 2.7; 97 % zeros 0.57 -> 0.44, 0.51 -> 0.43, 0.46 -> 0.43, 0.46 -> 0.43, 1.15 -> 0.87; exp(4 N(0, 1)) 0.87 -> 0.79,
+// 0.65 -> 0.69, 0.77 -> 0.77, 1.6 -> 1.1, 1.5 -> 1.3; and no worse at any size of the overlap (the first three kinds).
+// What bias is left grows with the columns: mean error 0 for a few products, -0.4 units at 32 x 32, -0.9 at 64 x 64.
 //
 // As a matrix product.  One side's matrices (the "A side") are stacked to one tall matrix of rows;
 // lane (row of the product) g meets row y of a matrix B of the other side with its row g + y.  Walking
@@ -25,16 +33,21 @@
 // are few, of rows y and y - 1 of the same one (nR = 2): lane g then stands for the stack's rows 2 g and
 // 2 g + 1, which meet row y - rho in the same A row 2 g + y, and the A rows are staged even and odd apart.
 //
-// Bound by shared memory: the products alone read it at 75..95 % of its rate, and what the drain warps and the
-// producers move comes on top; a wrapped row costs one to two thousand clocks that two result buffers hide in part.
+// Bound by shared memory: the products alone read it at 75..95 % of its rate, and beside them a warp gets one access in
+// about ten clocks; what the drain warps and the producers move comes on top.  A wrapped row costs the warp about 250
+// clocks and 5 a column.  Two sums of 128 columns in two buffers fill tensor memory.  256 columns halve what the
+// products read of A per result and leave room for one buffer: there the small products' sums stay in tensor memory
+// from row to row and are fetched only where a lane wraps, and a row's large products, issued last, wait until those
+// of the row before have been drained (48 x 48 16 x 2048 350 -> 296 us, 64 x 64 1 x 512 161 -> 152).
 // Tried and left: writing a wrapped row from its lane's registers straight to global memory (one 4-byte store in
 // flight per SM every 7 clocks: 64 x 64 1 x 512 took 327 us), 4 and 16 matrices interleaved (fewer wraps, but all
-// warps wait for the one that writes: 32 x 32 32 x 64 88 us against 70).
-// Measured on B200 (us, tile kernel -> this one): 256 x 256 one pair 168 -> 94, 64 x 64 1 x 512 353 -> 121,
-// 32 x 32 32 x 64 101 -> 69, 48 x 48 16 x 2048 450 -> 205, 27 x 43 9 x 35 53 -> 33, 256 x 256 1 x 32 4657 -> 1609.
+// warps wait for the one that writes: 32 x 32 32 x 64 88 us against 70), one sum of row totals h + small instead of two
+// (sparse operands off by 0.51..0.63 units, FFMAs 0.46..0.57).
+// Measured on B200 (us, tile kernel -> this one): 256 x 256 one pair 168 -> 107, 64 x 64 1 x 512 353 -> 153,
+// 32 x 32 32 x 64 102 -> 84, 48 x 48 16 x 2048 449 -> 296, 27 x 43 9 x 35 54 -> 33, 256 x 256 1 x 32 4655 -> 1904.
 //
-// Roles of a block (12 warps): warps 0..7 drain tensor memory into register sums and write results,
-// 8..10 build the Toeplitz rows, warp 11 issues the matrix products.
+// Roles of a block: the first 8 or 16 warps drain tensor memory into register sums and write results, three build the
+// Toeplitz rows, the last one issues the matrix products.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -49,10 +62,7 @@ namespace xcorr {
 
 namespace {
 
-constexpr int kDrainWarps = 8, kProducerWarps = 3;
-constexpr int kMmaWarp = kDrainWarps + kProducerWarps;
-constexpr int kThreads = 32 * (kMmaWarp + 1);
-static_assert(kThreads == kTensorThreads, "block size");
+constexpr int kProducerWarps = 3;
 constexpr int kProducers = 32 * kProducerWarps;
 constexpr int kRowRing = 4;                            // split rows of a B matrix kept by the producers
 constexpr int kRowElems = kTensorMaxRow / kProducers;  // elements of a step's rows per producer thread
@@ -103,7 +113,7 @@ __device__ __forceinline__ void tc_commit(uint32_t bar) {
 }
 // KEEP: what becomes of the A operand in the tensor core's collector buffer -- read and kept for the next
 // product (fill), taken from there for the last time (lastuse), or neither.
-enum Keep { kDiscard, kFill, kLastUse };
+enum Keep { kDiscard, kFill, kUse, kLastUse };
 #define XC_MMA(OP) \
     asm volatile("{ .reg .pred p; .reg .b64 a, b;\n\t" \
                  "mov.b64 a, {%1, %3};\n\t" \
@@ -114,25 +124,26 @@ enum Keep { kDiscard, kFill, kLastUse };
 template<Keep KEEP = kDiscard>
 __device__ __forceinline__ void tc_mma(uint32_t d, uint32_t a_lo, uint32_t b_lo, uint32_t desc_hi, uint32_t idesc, uint32_t accumulate) {
     if (KEEP == kFill) XC_MMA("fill");
+    else if (KEEP == kUse) XC_MMA("use");
     else if (KEEP == kLastUse) XC_MMA("lastuse");
     else XC_MMA("discard");
 }
 #undef XC_MMA
 // Asynchronous: the registers are the caller's after tc_load_wait.
-__device__ __forceinline__ void tc_load(uint32_t addr, uint32_t (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                 : "r"(addr));
+__device__ __forceinline__ void tc_load(uint32_t addr, uint32_t (&r)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]) : "r"(addr));
 }
 // (the registers pass through it, so that nothing reads them earlier)
-__device__ __forceinline__ void tc_load_wait(uint32_t (&r)[16]) {
+__device__ __forceinline__ void tc_load_wait(uint32_t (&r)[8]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
-                 :: "memory");
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]) :: "memory");
 }
+__device__ __forceinline__ void tc_store(uint32_t addr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 :: "r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+__device__ __forceinline__ void tc_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // Results are written once and never read here; without a memory clobber the compiler may keep the
 // shared-memory loads of the next ones in front.
 __device__ __forceinline__ void put_result(float* to, float v, bool add) {
@@ -172,7 +183,7 @@ struct Step {
 };
 
 struct Shared {
-    unsigned long long b_full[kTensorMaxSlots], b_empty[kTensorMaxSlots], d_full[2], d_empty[2], drained;
+    unsigned long long b_full[kTensorMaxSlots], b_empty[kTensorMaxSlots], d_full[2], d_empty[2], rest_free[2], drained;
     uint32_t tmem;
     int gave_up;
     int n_steps;
@@ -183,7 +194,7 @@ struct Shared {
     Step step[kMaxSteps];
     // a drain warp's columns in the order they are written, neighbours in a result row one after the other
     // (by Toeplitz matrix, then x shift): column, and its place in its output row's image; INT_MIN: no result
-    int2 column[2 * kTensorMaxCols];
+    int2 column[kTensorMaxCols];
     long long row_end[2][128];                     // the output rows of a drain lane's last sums
     long long row_out[2][2][128];                  // a stack row's output rows before / after its wrap, per rho and lane; -1: none
 };
@@ -207,7 +218,7 @@ __device__ __noinline__ void direct_block(const TensorArgs& args, const BlockTas
     const int H = p.H, W = p.W, OW = 2 * W - 1, OH = 2 * H - 1;
     const int groups8 = p.DW / 8 * p.nB;
     const int total = 128 * p.nR * 2 * groups8;
-    for (int idx = threadIdx.x; idx < total; idx += kThreads) {
+    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
         const int g8 = idx % groups8, row = idx / groups8;
         const int srow = t.row0 + (row >> 1) / p.J, wrapped = row & 1;
         const int b = g8 % p.nB, sx0 = t.sx_lo + g8 / p.nB * 8;
@@ -247,19 +258,23 @@ __device__ __noinline__ void direct_block(const TensorArgs& args, const BlockTas
     }
 }
 
-// NC: result columns per drain warp (half of the block's).  NR: rows of a B matrix taken together; with
+// D: result columns of the block, NC for every four drain warps.  NR: rows of a B matrix taken together; with
 // two, the 8-column groups belong to row offsets 0 and 1 in turn.
 // MANY: the A side's columns are staged in more than one chunk (a build of its own: the sums then stay in
 // registers across the whole block's code, which the single chunk's warps would pay for with spills).
-template<int NC, int NR, bool MANY>
-__global__ void __launch_bounds__(kThreads, 1) tensor_kernel(const __grid_constant__ TensorArgs args) {
+template<int D, int NR, bool MANY>
+__global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __grid_constant__ TensorArgs args) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ Shared sh;
     const TensorPlan& p = args.p;
     const int H = p.H, W = p.W, OW = 2 * W - 1, OH = 2 * H - 1;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    constexpr int D = 2 * NC;                                    // result columns of a buffer
-    constexpr uint32_t kTmemCols = D <= 64 ? 128 : D <= 128 ? 256 : 512;
+    constexpr int kDrainWarps = kTensorDrainWarps<D>, NC = 4 * D / kDrainWarps, kMmaWarp = kDrainWarps + kProducerWarps, kThreads = kTensorThreads<D>;
+    static_assert(kThreads == 32 * (kMmaWarp + 1), "block size");
+    // Up to 128 columns tensor memory has two buffers for the sums of either kind, drained after every row.  256 columns
+    // fill it with one: the small products' sums then stay in it, and a warp fetches them only where one of its lanes wraps.
+    constexpr bool kResident = D == 256;
+    constexpr uint32_t kTmemCols = kResident ? 2 * D : 4 * D;
 
     // ---- the block's task: x-shift tiles outermost, the heaviest (around shift 0) first
     BlockTask t;
@@ -302,7 +317,11 @@ __global__ void __launch_bounds__(kThreads, 1) tensor_kernel(const __grid_consta
     if (tid == 0) {
         sh.gave_up = 0; sh.bad = 0;
         for (int i = 0; i < p.slots; ++i) { bar_init(smem_addr(&sh.b_full[i]), kProducers); bar_init(smem_addr(&sh.b_empty[i]), 1); }
-        for (int i = 0; i < 2; ++i) { bar_init(smem_addr(&sh.d_full[i]), 1); bar_init(smem_addr(&sh.d_empty[i]), 32 * kDrainWarps); }
+        for (int i = 0; i < 2; ++i) {
+            bar_init(smem_addr(&sh.d_full[i]), 1);
+            bar_init(smem_addr(&sh.d_empty[i]), kDrainWarps);
+            bar_init(smem_addr(&sh.rest_free[i]), kDrainWarps);
+        }
         bar_init(smem_addr(&sh.drained), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -364,11 +383,14 @@ __global__ void __launch_bounds__(kThreads, 1) tensor_kernel(const __grid_consta
     int pass = 0;                                  // chunks walked
     // The chunks are walked to and fro: a stack row that does not wrap on the way keeps its sums from chunk
     // to chunk, one that does writes them at its turning point once per chunk (added from the third time on).
-    float sum[NC];
-    if (MANY) {
+    // Sums of the large products and of the small ones: added to each other once, when a result is written.
+    // (`rest` of the 256-column build stands in tensor memory)
+    float sum[NC], rest[kResident ? 1 : NC];
+    const auto no_sums = [&] {
 #pragma unroll
-        for (int c = 0; c < NC; ++c) sum[c] = 0.f;
-    }
+        for (int c = 0; c < NC; ++c) { sum[c] = 0.f; if (!kResident) rest[c] = 0.f; }
+    };
+    if (MANY) no_sums();
     bool ok = true;
     for (int k0 = 0; k0 < p.Kp; k0 += p.KC) {
         const int kc = min(p.KC, p.Kp - k0);
@@ -441,66 +463,124 @@ __global__ void __launch_bounds__(kThreads, 1) tensor_kernel(const __grid_consta
         const int back = MANY ? pass & 1 : 0;
         if (warp < kDrainWarps) {
             // ================= drain: tensor memory -> register sums -> results
-            if (!MANY) {
-#pragma unroll
-                for (int c = 0; c < NC; ++c) sum[c] = 0.f;
-            }
+            if (!MANY) no_sums();
             const uint32_t t_addr = tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)half_col;
-            for (int i = 0; ok && i < steps_y; ++i) {
-                const unsigned it = it_base + i;
-                // stack rows that run on into the next matrices with this step: their sums so far are result
-                // rows, written by the whole warp (J lanes wrap at a time), and the next sums start from zero
+            // Stack rows that run on into the next matrices with step i: their sums so far are result rows, and the
+            // next ones start from zero.
+            unsigned who0 = 0, who1 = 0;
+            const auto wrap_at = [&](int i) {
                 const int turn = back ? steps_y - i : i;       // (backwards, the rows come back with the step before)
-                const unsigned who0 = __ballot_sync(0xffffffffu, turn == wrap_step[0]);
-                const unsigned who1 = NR == 2 ? __ballot_sync(0xffffffffu, turn == wrap_step[NR - 1]) : 0u;
-                const unsigned who = who0 | who1;
-                const float keep0 = who0 >> lane & 1 ? 0.f : 1.f, keep1 = who1 >> lane & 1 ? 0.f : 1.f;
+                who0 = __ballot_sync(0xffffffffu, turn == wrap_step[0]);
+                who1 = NR == 2 ? __ballot_sync(0xffffffffu, turn == wrap_step[NR - 1]) : 0u;
                 if (who0 >> lane & 1) wrapped[0] = !back;
                 if (NR == 2 && (who1 >> lane & 1)) wrapped[NR - 1] = !back;
-                for (unsigned rest = who; rest;) {
-                    // (more than one group of J lanes where a warp's stack rows span more than H)
-                    const unsigned group = ((1u << p.J) - 1u) << ((__ffs(rest) - 1) & ~(p.J - 1)), now = rest & group;
-                    rest &= ~group;
-                    if (now >> lane & 1) {
-                        float4* to = reinterpret_cast<float4*>(scratch + lane % p.J * (NC + 4));
+            };
+            // result rows of the lanes in `now`, which stand in the warp's scratch space, written by the whole warp
+            const auto write_rows = [&](unsigned now) {
+                __syncwarp();
 #pragma unroll
-                        for (int c = 0; c < NC; c += 4) to[c / 4] = make_float4(sum[c], sum[c + 1], sum[c + 2], sum[c + 3]);
-                    }
-                    __syncwarp();
+                for (int z = 0; z < NC / 32; ++z) {
                     // (with two rows taken together the first half of the order belongs to row offset 0)
-                    const int2* column = &sh.column[half_col + lane];
-                    int2 col[NC / 32];
-#pragma unroll
-                    for (int z = 0; z < NC / 32; ++z) col[z] = column[32 * z];
+                    const int2 col = sh.column[half_col + 32 * z + lane];
+                    const bool second = NR == 2 && 32 * z + lane >= NC / 2;
                     for (unsigned left = now; left; left &= left - 1) {
                         const int src = __ffs(left) - 1;
-                        const float* from = scratch + src % p.J * (NC + 4);
-                        const long long off0 = who0 >> src & 1 ? sh.row_out[back][0][(warp & 3) * 32 + src] : -1;
-                        const long long off1 = NR == 2 && (who1 >> src & 1) ? sh.row_out[back][NR - 1][(warp & 3) * 32 + src] : -1;
-                        float v[NC / 32];
-#pragma unroll
-                        for (int z = 0; z < NC / 32; ++z) v[z] = from[col[z].x];
-#pragma unroll
-                        for (int z = 0; z < NC / 32; ++z) {
-                            const long long off = NR == 2 && 32 * z + lane >= NC / 2 ? off1 : off0;
-                            if (off >= 0 && col[z].y != INT_MIN) put_result(t.out + off + col[z].y, v[z], MANY && pass >= 2);
-                        }
+                        const long long off = (second ? who1 : who0) >> src & 1 ? sh.row_out[back][second ? NR - 1 : 0][(warp & 3) * 32 + src] : -1;
+                        const float v = scratch[src % p.J * (NC + 4) + col.x];
+                        if (off >= 0 && col.y != INT_MIN) put_result(t.out + off + col.y, v, MANY && pass >= 2);
                     }
-                    __syncwarp();
                 }
-                ok = bar_wait(smem_addr(&sh.d_full[it & 1]), (it >> 1) & 1, &sh.gave_up);
+                __syncwarp();
+            };
+            float4* mine = reinterpret_cast<float4*>(scratch + lane % p.J * (NC + 4));
+            for (int i = 0; ok && i < steps_y; ++i) {
+                const unsigned it = it_base + i;
+                if (!kResident) {
+                    wrap_at(i);
+                    for (unsigned todo = who0 | who1; todo;) {
+                        // (more than one group of J lanes where a warp's stack rows span more than H)
+                        const unsigned now = todo & ((1u << p.J) - 1u) << ((__ffs(todo) - 1) & ~(p.J - 1));
+                        todo &= ~now;
+                        if (now >> lane & 1) {
+#pragma unroll
+                            for (int c = 0; c < NC; c += 4)
+                                mine[c / 4] = make_float4(sum[c] + rest[kResident ? 0 : c], sum[c + 1] + rest[kResident ? 0 : c + 1],
+                                                          sum[c + 2] + rest[kResident ? 0 : c + 2], sum[c + 3] + rest[kResident ? 0 : c + 3]);
+                        }
+                        write_rows(now);
+                    }
+                }
+                const int buffer = kResident ? 0 : it & 1;
+                if (kResident) {
+                    // The next row's small products may be added to the sums that stay in tensor memory (rest_free) once the
+                    // lanes that wrap with it have taken theirs: at once where there are none.  Two barriers in turn: a warp
+                    // can be a row ahead of the products here, not two (d_full of this row comes before the row after next).
+                    if (i + 1 < steps_y) wrap_at(i + 1); else who0 = who1 = 0;
+                    if (!(who0 | who1) && lane == 0) bar_arrive(smem_addr(&sh.rest_free[it & 1]));
+                }
+                ok = bar_wait(smem_addr(&sh.d_full[buffer]), (kResident ? it : it >> 1) & 1, &sh.gave_up);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
+                if (kResident) {
 #pragma unroll
-                for (int c0 = 0; c0 < NC; c0 += 16) {
-                    uint32_t v[16];
-                    tc_load(t_addr + (it & 1) * D + c0, v);
-                    tc_load_wait(v);
-                    if (c0 + 16 >= NC) { tc_fence_before(); bar_arrive(smem_addr(&sh.d_empty[it & 1])); }
+                    for (int c0 = 0; c0 < NC; c0 += 16) {
+                        uint32_t v[8], w[8];
+                        tc_load(t_addr + c0, v);
+                        tc_load(t_addr + c0 + 8, w);
+                        tc_load_wait(v);
+                        tc_load_wait(w);
 #pragma unroll
-                    for (int c = 0; c < 16; ++c)
-                        sum[c0 + c] = fmaf(sum[c0 + c], NR == 2 && (c & 8) ? keep1 : keep0, __uint_as_float(v[c]));   // (exact: times 1 or 0)
+                        for (int c = 0; c < 8; ++c) { sum[c0 + c] += __uint_as_float(v[c]); sum[c0 + 8 + c] += __uint_as_float(w[c]); }
+                    }
+                    // Lanes that wrap with the next row (one group of J at most, by the plan).  No products run until this is
+                    // done: beside them a warp gets one access to shared memory in about ten clocks.
+                    if (who0 | who1) {
+#pragma unroll
+                        for (int c0 = 0; c0 < NC; c0 += 8) {
+                            const unsigned who = NR == 2 && (c0 & 8) ? who1 : who0;      // (eight columns belong to one row offset)
+                            if (!who) continue;
+                            uint32_t w[8];
+                            tc_load(t_addr + D + c0, w);
+                            tc_load_wait(w);
+                            if (who >> lane & 1) {
+                                float f[8];
+#pragma unroll
+                                for (int c = 0; c < 8; ++c) { f[c] = sum[c0 + c] + __uint_as_float(w[c]); sum[c0 + c] = 0.f; w[c] = 0u; }
+                                mine[c0 / 4] = make_float4(f[0], f[1], f[2], f[3]);
+                                mine[c0 / 4 + 1] = make_float4(f[4], f[5], f[6], f[7]);
+                            }
+                            tc_store(t_addr + D + c0, w);
+                        }
+                        tc_store_wait();
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (who0 | who1) bar_arrive(smem_addr(&sh.rest_free[it & 1]));
+                        bar_arrive(smem_addr(&sh.d_empty[0]));
+                    }
+                    if (who0 | who1) write_rows(who0 | who1);
+                } else {
+                    const float keep0 = who0 >> lane & 1 ? 0.f : 1.f, keep1 = who1 >> lane & 1 ? 0.f : 1.f;
+#pragma unroll
+                    for (int c0 = 0; c0 < NC; c0 += 8) {
+                        uint32_t v[8], w[8];
+                        tc_load(t_addr + buffer * 2 * D + c0, v);
+                        tc_load(t_addr + buffer * 2 * D + D + c0, w);
+                        tc_load_wait(v);
+                        tc_load_wait(w);
+                        // (eight columns belong to one row offset; exact: times 1 or 0)
+                        const float keep = NR == 2 && (c0 & 8) ? keep1 : keep0;
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) {
+                            sum[c0 + c] = fmaf(sum[c0 + c], keep, __uint_as_float(v[c]));
+                            rest[kResident ? 0 : c0 + c] = fmaf(rest[kResident ? 0 : c0 + c], keep, __uint_as_float(w[c]));
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(smem_addr(&sh.d_empty[buffer]));
                 }
             }
         } else if (warp < kMmaWarp) {
@@ -582,6 +662,7 @@ __global__ void __launch_bounds__(kThreads, 1) tensor_kernel(const __grid_consta
                 fence_async();
                 bar_arrive(smem_addr(&sh.b_full[slot]));
             }
+            if (MANY) no_sums();                      // (the other roles keep no registers for them)
         } else {
             // ================= matrix products: one row of B against 128 rows of A
             const bool leader = elect_one();
@@ -597,40 +678,60 @@ __global__ void __launch_bounds__(kThreads, 1) tensor_kernel(const __grid_consta
                 const unsigned it = it_base + i, use = it / p.slots;
                 const int slot = (int)(it - use * p.slots);
                 ok = bar_wait(smem_addr(&sh.b_full[slot]), use & 1, &sh.gave_up);
-                if (ok && it >= 2) ok = bar_wait(smem_addr(&sh.d_empty[it & 1]), ((it >> 1) - 1) & 1, &sh.gave_up);
+                if (kResident && ok && it >= 1) ok = bar_wait(smem_addr(&sh.rest_free[(it - 1) & 1]), ((it - 1) >> 1) & 1, &sh.gave_up);
+                if (!kResident && ok && it >= 2) ok = bar_wait(smem_addr(&sh.d_empty[it & 1]), ((it >> 1) - 1) & 1, &sh.gave_up);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
+                const int place = back ? steps_y - 1 - i : i;
+                const uint32_t a0 = a_lo0 + ((place % NR) * res_rows + place / NR) * p.J;
+                const uint32_t large = tmem + (kResident ? 0 : it & 1) * 2 * D, small = large + D;
+                const uint32_t b0 = ((b_base + slot * slot_bytes) >> 4) | lbo_b;
+                // The first product of a row into either sum spans all result columns (against the Toeplitz matrix's
+                // zeros outside its window) and overwrites the buffer; the sums that stay there start with the first row.
                 if (leader) {
-                    const int place = back ? steps_y - 1 - i : i;
-                    const uint32_t a0 = a_lo0 + ((place % NR) * res_rows + place / NR) * p.J, d0 = tmem + (it & 1) * D;
-                    const uint32_t b0 = ((b_base + slot * slot_bytes) >> 4) | lbo_b;
-                    // the products of the small parts first: they lose nothing beside the sum of the large ones.
-                    // The row's first product spans all result columns (against the Toeplitz matrix's zeros
-                    // outside its window) and overwrites the buffer.
-                    tc_mma(d0, a0 + st[0].a_off + 2 * a_part16, b0 + first_off, desc_hi, idesc_all, 0);
+                    tc_mma(small, a0 + st[0].a_off + 2 * a_part16, b0 + first_off, desc_hi, idesc_all, kResident && it > 0);
 #pragma unroll
                     for (int s = 0; s < kMaxSteps; ++s) {
                         if (s >= n_steps) break;
-                        const uint32_t a = a0 + st[s].a_off, b = b0 + st[s].b_off, d = d0 + st[s].d_off, id = st[s].idesc;
+                        const uint32_t a = a0 + st[s].a_off, b = b0 + st[s].b_off, d = small + st[s].d_off, id = st[s].idesc;
                         if (s > 0) tc_mma(d, a + 2 * a_part16, b, desc_hi, id, 1);
-                        // (the middle and the high part of A are each read once for two products: 27 x 43 9 x 35 34.7 ->
-                        // 32.8 us, one 256 x 256 pair 95.8 -> 94.2; nothing where the wrapped rows set the pace)
+                        // (the middle and the high part of A are each read once for two products or three)
                         tc_mma<kFill>(d, a + a_part16, b + bp, desc_hi, id, 1);
                         tc_mma<kLastUse>(d, a + a_part16, b, desc_hi, id, 1);
                         tc_mma<kFill>(d, a, b + 2 * bp, desc_hi, id, 1);
-                        tc_mma<kLastUse>(d, a, b + bp, desc_hi, id, 1);
+                        if (kResident || s == 0) {
+                            tc_mma<kLastUse>(d, a, b + bp, desc_hi, id, 1);
+                        } else {
+                            tc_mma<kUse>(d, a, b + bp, desc_hi, id, 1);
+                            tc_mma<kLastUse>(large + st[s].d_off, a, b, desc_hi, id, 1);
+                        }
+                        if (!kResident && s == 0) tc_mma(large, a, b0 + first_off, desc_hi, idesc_all, 0);
                     }
+                }
+                __syncwarp();
+                if (kResident) {
+                    // the large products last: their sums of the row before are drained meanwhile
+                    if (it >= 1) ok = bar_wait(smem_addr(&sh.d_empty[0]), (it - 1) & 1, &sh.gave_up);
+                    ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (leader) {
+                        tc_mma(large, a0 + st[0].a_off, b0 + first_off, desc_hi, idesc_all, 0);
 #pragma unroll
-                    for (int s = 0; s < kMaxSteps; ++s) {
-                        if (s >= n_steps) break;
-                        tc_mma(d0 + st[s].d_off, a0 + st[s].a_off, b0 + st[s].b_off, desc_hi, st[s].idesc, 1);
+                        for (int s = 1; s < kMaxSteps; ++s) {
+                            if (s >= n_steps) break;
+                            tc_mma(large + st[s].d_off, a0 + st[s].a_off, b0 + st[s].b_off, desc_hi, st[s].idesc, 1);
+                        }
                     }
+                }
+                if (leader) {
                     tc_commit(smem_addr(&sh.b_empty[slot]));
-                    tc_commit(smem_addr(&sh.d_full[it & 1]));
+                    tc_commit(smem_addr(&sh.d_full[kResident ? 0 : it & 1]));
                 }
                 __syncwarp();
             }
+            if (MANY) no_sums();
         }
         it_base += steps_y;
         ++pass;
@@ -644,7 +745,19 @@ __global__ void __launch_bounds__(kThreads, 1) tensor_kernel(const __grid_consta
     // products have completed), 16 lanes at a time, so that a store instruction writes up to 32 neighbours.
     if (ok && warp < kDrainWarps) {
         float* tile = reinterpret_cast<float*>(smem) + warp * 16 * (NC + 1);
-        // (both halves of a warp's columns set the same values)
+        if (kResident) {
+            const uint32_t t_addr = tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)half_col + D;
+#pragma unroll
+            for (int c0 = 0; c0 < NC; c0 += 8) {
+                uint32_t w[8];
+                tc_load(t_addr + c0, w);
+                tc_load_wait(w);
+#pragma unroll
+                for (int c = 0; c < 8; ++c) sum[c0 + c] += __uint_as_float(w[c]);
+            }
+            tc_fence_before();
+        }
+        // (the warps of the same lanes set the same values)
         unsigned again[NR];                        // rows that wrapped on the way have been written before, unless this was the only pass
 #pragma unroll
         for (int rho = 0; rho < NR; ++rho) {
@@ -655,7 +768,7 @@ __global__ void __launch_bounds__(kThreads, 1) tensor_kernel(const __grid_consta
         for (int half = 0; half < 2; ++half) {
             if (lane >> 4 == half) {
 #pragma unroll
-                for (int c = 0; c < NC; ++c) tile[(lane & 15) * (NC + 1) + c] = sum[c];
+                for (int c = 0; c < NC; ++c) tile[(lane & 15) * (NC + 1) + c] = kResident ? sum[c] : sum[c] + rest[kResident ? 0 : c];
             }
             __syncwarp();
 #pragma unroll 1
@@ -724,19 +837,19 @@ int up(int v, int m) { return (v + m - 1) / m * m; }
 }  // namespace
 
 cudaError_t launch_tensor(const TensorArgs& a, int device, cudaStream_t stream) {
-    void (*const kernels[2][2][4])(TensorArgs) = {
-        {{tensor_kernel<32, 1, false>, tensor_kernel<64, 1, false>, tensor_kernel<96, 1, false>, tensor_kernel<128, 1, false>},
-         {tensor_kernel<32, 1, true>, tensor_kernel<64, 1, true>, tensor_kernel<96, 1, true>, tensor_kernel<128, 1, true>}},
-        {{tensor_kernel<32, 2, false>, tensor_kernel<64, 2, false>, tensor_kernel<96, 2, false>, tensor_kernel<128, 2, false>},
-         {tensor_kernel<32, 2, true>, tensor_kernel<64, 2, true>, tensor_kernel<96, 2, true>, tensor_kernel<128, 2, true>}}};
-    const int many = a.p.Kp > a.p.KC ? 1 : 0, cols = a.p.NC / 32 - 1;
+    void (*const kernels[2][2][3])(TensorArgs) = {
+        {{tensor_kernel<64, 1, false>, tensor_kernel<128, 1, false>, tensor_kernel<256, 1, false>},
+         {tensor_kernel<64, 1, true>, tensor_kernel<128, 1, true>, tensor_kernel<256, 1, true>}},
+        {{tensor_kernel<64, 2, false>, tensor_kernel<128, 2, false>, tensor_kernel<256, 2, false>},
+         {tensor_kernel<64, 2, true>, tensor_kernel<128, 2, true>, tensor_kernel<256, 2, true>}}};
+    const int many = a.p.Kp > a.p.KC ? 1 : 0, cols = a.p.D / 128;
     auto* kernel = kernels[a.p.nR - 1][many][cols];
-    static SmemLimit limits[2][2][4];
+    static SmemLimit limits[2][2][3];
     const cudaError_t e = limits[a.p.nR - 1][many][cols].allow(device, a.p.smem_bytes, [&](size_t bytes) {
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     });
     if (e != cudaSuccess) return e;
-    kernel<<<a.p.grid, kThreads, a.p.smem_bytes, stream>>>(a);
+    kernel<<<a.p.grid, tensor_threads(a.p.D), a.p.smem_bytes, stream>>>(a);
     return cudaGetLastError();
 }
 
@@ -747,7 +860,7 @@ cudaError_t tensor_wait_timeouts(unsigned* count) {
     return e;
 }
 
-bool plan_tensor(const PairMap& pm, int H, int W, int sm_count, int max_slices, TensorPlan* out, double* out_us) {
+bool plan_tensor(const PairMap& pm, int H, int W, int sm_count, int max_slices, double max_err2, TensorPlan* out, double* out_us) {
     if (H < 8 || W < 8 || H > 1024 || W > kTensorMaxRow) return false;
     const bool shared_rights = pm.n_left == 1 || pm.right_stride == 0;     // every left meets every right
     double best = 1e30;
@@ -767,7 +880,7 @@ bool plan_tensor(const PairMap& pm, int H, int W, int sm_count, int max_slices, 
         }
         if ((long long)p.nA * H > 1 << 30) continue;
         p.Kp = up(W, 16);
-        for (int NC = 32; NC <= kTensorMaxCols; NC += 32)
+        for (int D = 64; D <= kTensorMaxCols; D *= 2)
         for (int nB = 1; nB <= std::min(p.nBt, kTensorMaxB); ++nB)
         for (int nR = 1; nR <= (nB == 1 ? 2 : 1); ++nR)
         for (int J = 1; J <= std::min(p.nA, kTensorMaxJ); J *= 2)
@@ -775,9 +888,9 @@ bool plan_tensor(const PairMap& pm, int H, int W, int sm_count, int max_slices, 
             if (S > 1 && (flip || p.nA != 1)) break;
             if (nB * W > kTensorMaxRow) continue;
             const int nS = nB * nR;
-            const int dw = 2 * NC / nS / 16 * 16;
+            const int dw = D / nS / 16 * 16;
             if (dw < 16) break;
-            p.NC = NC; p.nB = nB; p.nR = nR; p.S = S; p.J = J;
+            p.D = D; p.nB = nB; p.nR = nR; p.S = S; p.J = J;
             p.stack_rows = (p.nA + J - 1) / J * H;
             p.m_tiles = (unsigned)((p.stack_rows + 128 / J * nR - 1) / (128 / J * nR));
             p.x_tiles = (2 * W - 1 + dw - 1) / dw;
@@ -791,9 +904,13 @@ bool plan_tensor(const PairMap& pm, int H, int W, int sm_count, int max_slices, 
             // Toeplitz rows of a step, whatever the tile
             if (((W + 13) / 8 + 1) * nS * 8 > kTensorMaxItems) continue;
             if (((128 / J * nR + 2 * H + rows) / H + 1) * J > kTensorMaxStack) continue;
+            const int drain_warps = tensor_threads(D) / 32 - 4, NC = 4 * D / drain_warps;
+            // (256 columns: one group of J lanes of a warp at most wraps at a time -- groups g and g' do together where
+            // nR * (g - g') is a multiple of H)
+            if (D == 256 && 32 / J > H / (H % nR == 0 ? nR : 1)) continue;
             const auto smem_of = [&] {
-                const size_t a_bytes = std::max<size_t>((size_t)3 * (p.KC / 8) * p.AR * 16, (size_t)kDrainWarps * 16 * (NC + 1) * 4);
-                return a_bytes + (size_t)p.slots * 3 * ((p.DW + p.KC) / 8) * nS * 128 + (size_t)kDrainWarps * J * (NC + 4) * 4 +
+                const size_t a_bytes = std::max<size_t>((size_t)3 * (p.KC / 8) * p.AR * 16, (size_t)drain_warps * 16 * (NC + 1) * 4);
+                return a_bytes + (size_t)p.slots * 3 * ((p.DW + p.KC) / 8) * nS * 128 + (size_t)drain_warps * J * (NC + 4) * 4 +
                        (size_t)12 * kRowRing * nB * p.row_words;
             };
             bool fits = false;
@@ -805,18 +922,29 @@ bool plan_tensor(const PairMap& pm, int H, int W, int sm_count, int max_slices, 
             if (!fits) continue;
             const int chunks = (p.Kp + p.KC - 1) / p.KC;
             p.KC = up((p.Kp + chunks - 1) / chunks, 16);
+            // (two rows together in 256 columns over several chunks: never within 5 % of the best plan timed)
+            if (D == 256 && nR == 2 && chunks > 1) continue;
+            // the sums in registers, one per row and chunk, taken one after the other in every slice (64 x 64: 1.97 measured,
+            // 2.05 by this; 256 x 256 in 37 slices 1.72, 1.61); rounding once and what the products leave out
+            const double sums = (double)H * chunks;
+            if (0.3 + 0.061 * (sums / ((double)S * S) + S) > max_err2) continue;
             // one block per SM: half of tensor memory or more, and the registers, are taken
             p.smem_bytes = std::max<size_t>(smem_of(), 120 * 1024);
             if ((double)nB * p.stride_b * (2.0 * H - 1) * (2.0 * W - 1) > 2e9) continue;    // (32-bit column offsets)
             const unsigned long long grid = (unsigned long long)p.x_tiles * p.groups * p.m_tiles * p.b_groups * S;
             if (grid > 0x7fffffffull) continue;
             p.grid = (unsigned)grid;
-            // time of a block in clocks: its matrix products at the tensor cores' rate or that of the
-            // shared memory they read, its drains, its Toeplitz rows; staging once per chunk
-            double sum_clk = 0, max_clk = 0;
+            // Time of a block in clocks: its matrix products at the tensor cores' rate or that of the shared memory they
+            // read, its Toeplitz rows, its drains and wrapped rows; of these the longest, and most of the second, since
+            // all of them share the memory.  Constants fitted to 2313 plans timed on 90 shapes (4 % in the mean square).
+            const double together = H % nR == 0 ? nR : 1;       // every so many steps several lanes of a block wrap at once
+            const double some = std::min(1.0 / together, 128.0 / J / H);                  // steps in which any does
+            const double wraps = some * std::max(1.0, 32.0 / J / H * together);           // groups of a warp, one after the other
+            const double wrap_clk = 248.0 + 5.3 * NC;
+            double sum_clk = 0, max_clk = 0, tile_clk[64];
             const int xt_n = std::min(p.x_tiles, 64);
             for (int xt = 0; xt < xt_n; ++xt) {
-                double clk = 4500.0 + 140.0 * NC;
+                double clk = 100.0 + 130.0 * D;
                 for (int k0 = 0; k0 < p.Kp; k0 += p.KC) {
                     const int kc = std::min(p.KC, p.Kp - k0);
                     const int X0 = p.Kp - 1 + W - 1 - xt * p.DW - k0;
@@ -825,28 +953,46 @@ bool plan_tensor(const PairMap& pm, int H, int W, int sm_count, int max_slices, 
                         const int lo = std::max(0, (X0 - W + 1 - 16 * s - 15) & ~7), hi = std::min(p.DW, X0 - 16 * s + 1);
                         if (hi <= lo) continue;
                         const double cols = (double)up(hi - lo, 16) * nS;
-                        row += 6 * std::max(cols / 2, 32 + cols / 4) + (row == 0 ? (p.DW * nS - cols) / 2 : 0);
+                        row += 6 * std::max(cols / 2, (D == 256 ? 21 : 16) + cols / 4) + (row == 0 ? p.DW * nS - cols : 0);
                     }
                     if (row == 0) continue;
                     const int blocks = std::min((W + 13) / 8 + 1, (p.DW + kc) / 8);
-                    const double produce = 440.0 + 210.0 * ((blocks * nS * 8 + kProducers - 1) / kProducers) + 80.0 * ((nB * W + kProducers - 1) / kProducers);
-                    // (a step waits for the slowest of the drain warps: some of them writes a wrapped row in most steps)
-                    const double drain = 110.0 + 3.7 * NC + (J == 1 ? 0.75 : 0.5) * std::min(1.0, 128.0 / J / H) * (300.0 + 9.0 * NC + 4.0 * J * NC);
-                    // (the 128-column build for several chunks spills in its producers)
-                    double c3[3] = {row + 40, p.Kp > p.KC && NC == 128 ? 1.6 * produce : produce, drain};
+                    double produce = 233.0 + 225.0 * ((blocks * nS * 8 + kProducers - 1) / kProducers) + 120.0 * ((nB * W + kProducers - 1) / kProducers);
+                    if (p.Kp > p.KC && D >= 128) produce += D == 128 ? 670.0 : 1540.0;    // (these builds spill)
+                    double drain = 6.4 * D;
+                    if (D == 256) {
+                        row = 0.95 * row + 15.0 + some * 830.0;
+                        drain += 0.57 * wraps * J * wrap_clk;
+                    } else {
+                        row = 0.95 * row + 40.0;
+                        drain += wraps * (1.0 + 0.16 * (J - 1)) * wrap_clk;
+                    }
+                    double c3[3] = {row, produce, drain};
                     std::sort(c3, c3 + 3);
-                    clk += (rows + nR - 1) * (c3[2] + 0.5 * c3[1]) + 3.0 * p.AR * (kc / 8) + 1500.0;
+                    clk += (rows + nR - 1) * (c3[2] + 0.66 * c3[1]) + 4.3 * p.AR * (kc / 8) + 6500.0;
                 }
+                tile_clk[xt] = clk;
                 sum_clk += clk;
                 max_clk = std::max(max_clk, clk);
             }
             const double total = sum_clk * ((double)p.grid / xt_n);
             const double waves = (double)p.grid / sm_count;
-            // the busiest SM: whole blocks
-            const double clk = p.x_tiles == 1 ? max_clk * (double)(long long)(waves + 0.999999)
-                                              : std::max(max_clk, total / sm_count + 0.5 * max_clk * (waves > 1));
-            double us = clk / 1850.0 + 7.0;
-            if (S > 1) us += 3.0 + (double)S * (2.0 * H - 1) * (2.0 * W - 1) * p.nBt * 4 / 4e6;
+            double us = 4.7;
+            if (S > 1) us += 2.0 + (double)S * (2.0 * H - 1) * (2.0 * W - 1) * p.nBt * 4 / 4e6;
+            if (us + std::max(max_clk, total / sm_count) / 1850.0 >= best) continue;
+            // the busiest SM: whole blocks, each to the SM that is free first, in the order of the launch (a tile's blocks are alike)
+            double clk = total / sm_count + 0.2 * max_clk;
+            if (waves <= 12 && p.x_tiles <= 64 && sm_count <= 256) {
+                double load[256] = {};
+                const int per_tile = (int)(p.grid / (unsigned)p.x_tiles), mid = (p.x_tiles - 1) / 2;
+                for (int o = 0; o < p.x_tiles; ++o) {
+                    const double c = tile_clk[(o & 1) ? mid + (o + 1) / 2 : mid - o / 2];
+                    for (int i = 0; i < sm_count; ++i) load[i] += c * (per_tile / sm_count + (i < per_tile % sm_count ? 1 : 0));
+                    if (per_tile % sm_count) std::sort(load, load + sm_count);
+                }
+                clk = *std::max_element(load, load + sm_count);
+            }
+            us += clk / 1850.0;
             if (us < best) { best = us; *out = p; }
         }
     }

@@ -2,6 +2,7 @@
 and its host-only entry points (planning, shard ranges, order helpers, argument checks that
 fail before any CUDA call) behave.  No kernel runs here."""
 import ctypes as C
+import math
 import os
 import re
 
@@ -152,10 +153,12 @@ def test_plans_exist_and_fit_for_a_sweep_of_shapes(xc):
                                  r"side=(left|right) matrices=(\d+) rows=(\d+) interleave=(\d+) x_tiles=(\d+) x_shifts=(\d+) "
                                  r"chunk=(\d+) slots=(\d+) S=(\d+) combine=(store|workspace)\}", text)
                 assert t, text
-                nc, grid, block, smem, H, W = (int(v) for v in t.groups()[:6])
+                D, grid, block, smem, H, W = (int(v) for v in t.groups()[:6])
                 nB, nR, J, x_tiles, dw, chunk, slots, S = (int(v) for v in t.groups()[7:15])
-                assert (H, W) == (rows, cols) and grid >= 1 and block == 384 and smem <= 227 * 1024, text
-                assert dw % 16 == 0 and dw * nB * nR <= 2 * nc and x_tiles * dw >= 2 * W - 1 and 16 <= chunk <= 64, text
+                assert (H, W) == (rows, cols) and grid >= 1 and block == {64: 384, 128: 640, 256: 640}[D] and smem <= 227 * 1024, text
+                assert dw % 16 == 0 and dw * nB * nR <= D and x_tiles * dw >= 2 * W - 1 and 16 <= chunk <= 64, text
+                # 256 columns: at most one group of a warp's stack rows wraps at a time
+                assert D < 256 or 32 // J <= H // math.gcd(H, nR), text
                 assert slots >= 2 and J in (1, 2) and (S > 1) == (t.group(16) == "workspace"), text
                 # (the workspace query answers for the tile plan of the shape, whose slices this plan shares)
                 text = xc.describe_plan(mode, rows, cols, nl, nr, xc.make_hints(kernel="tile"))

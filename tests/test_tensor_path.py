@@ -38,6 +38,17 @@ def test_small_calls_and_finer_sums_stay(xc, shape):
     assert "kernel=tensor" not in plan(xc, shape)
 
 
+# timed at least as fast on the tile kernel (us on one B200, tile kernel / tensor cores): few rows, of which several of a
+# warp wrap at once, and shapes whose blocks fill little more than a whole number of waves
+TILE_FASTER = [("one_to_many", 8, 158, 1, 411), ("one_to_many", 69, 68, 1, 67), ("n_to_m", 13, 72, 2, 1482), ("n_to_mn", 12, 94, 2, 752),   # 47/54 112/115 169/187 52/60
+               ("n_to_mn", 10, 148, 3, 387), ("one_to_many", 8, 85, 1, 781), ("one_to_many", 40, 200, 1, 30), ("n_to_mn", 93, 75, 59, 59)]   # 65/61 38/37 123/169 194/206
+
+
+@pytest.mark.parametrize("shape", TILE_FASTER)
+def test_calls_that_gain_nothing_stay(xc, shape):
+    assert plan(xc, shape).startswith("kernel=tile<")
+
+
 def run(xc, torch, shape, left, right, hints=None, workspace=True):
     mode, rows, cols, nl, nr = shape
     guard = 256

@@ -132,7 +132,6 @@ constexpr int kTensorMaxRow = 576;    // elements of one row of a block's B matr
 constexpr int kTensorMaxItems = 576;  // 8-element rows of the core matrices of a step
 constexpr int kTensorMaxCols = 256;   // result columns of a block
 constexpr int kTensorMaxJ = 2;        // A matrices interleaved row by row
-constexpr int kTensorMaxStack = 64;   // A matrices a block's rows can touch
 // instruction descriptor without its N: 32-bit accumulators, bfloat16 operands, both K-major, M = 128
 constexpr uint32_t kTensorIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (8u << 24);
 // drain warps for 32 rows and 32 columns each (256 columns: 64), three producer warps and one that issues the products

@@ -69,12 +69,26 @@ constexpr int kRowElems = kTensorMaxRow / kProducers;  // elements of a step's r
 constexpr int kMaxItems = kTensorMaxItems / kProducers;  // Toeplitz rows of a step per producer thread
 constexpr int kMaxSteps = kTensorMaxChunk / 16;
 
-// Operands whose largest magnitude lies outside [2^-60, 2^50) (and infinities and NaN) are not
-// multiplied as three bfloat16 parts: the smallest part of a value below 2^-110 has no bits left, and
-// products of parts must neither overflow nor meet the Toeplitz matrix's zeros as infinities.
-constexpr unsigned kLargeBits = 0x58800000u, kSmallBits = 0x21800000u;
-__device__ __forceinline__ bool out_of_range(unsigned max_bits) {
-    return max_bits >= kLargeBits || (max_bits != 0 && max_bits < kSmallBits);
+// Operands that are not multiplied as three bfloat16 parts, by the magnitudes of the elements a block meets:
+// infinities, NaN and 2^50 upwards (products of parts must neither overflow nor meet the Toeplitz matrix's zeros as
+// infinities); below 2^-110 the last part runs out of bits; and where the smallest elements of both sides have a
+// product below 2^-100, products of parts can fall under the smallest normal number.  (Zeros are exact.)
+constexpr unsigned kLargeBits = 0x58800000u, kTinyBits = 0x08800000u;
+struct Magnitudes { unsigned large, small; };        // bits of the largest magnitude and of the smallest that is not zero
+constexpr Magnitudes kNoMagnitudes = {0u, 0x7f800000u};
+__device__ __forceinline__ void see(Magnitudes& m, unsigned bits) {
+    bits &= 0x7fffffffu;
+    m.large = max(m.large, bits);
+    m.small = min(m.small, bits - 1u);               // (a zero becomes the largest number there is)
+}
+__device__ __forceinline__ void merge(Magnitudes* of_block, Magnitudes m) {
+    m.large = __reduce_max_sync(0xffffffffu, m.large);
+    m.small = __reduce_min_sync(0xffffffffu, m.small);
+    if ((threadIdx.x & 31) == 0) { atomicMax(&of_block->large, m.large); atomicMin(&of_block->small, m.small); }
+}
+__device__ __forceinline__ bool out_of_range(const Magnitudes& a, const Magnitudes& b) {
+    const unsigned least = min(a.small, b.small) + 1u;
+    return max(a.large, b.large) >= kLargeBits || least < kTinyBits || ((a.small + 1u) >> 23) + ((b.small + 1u) >> 23) < 2u * 127u - 100u;
 }
 
 __device__ unsigned g_tensor_timeouts = 0;
@@ -188,9 +202,7 @@ struct Shared {
     int gave_up;
     int n_steps;
     uint32_t first_off;  // B operand of the chunk's first product, which spans all result columns
-    unsigned bad;
-    unsigned b_max[kTensorMaxB];
-    unsigned a_max[kTensorMaxStack];
+    Magnitudes a_mag, b_mag;
     Step step[kMaxSteps];
     // a drain warp's columns in the order they are written, neighbours in a result row one after the other
     // (by Toeplitz matrix, then x shift): column, and its place in its output row's image; INT_MIN: no result
@@ -315,7 +327,8 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
     float* scratch = reinterpret_cast<float*>(smem + (ring_base - a_base) + 12 * ring_words) + (warp < kDrainWarps ? warp * scratch_words : 0);
 
     if (tid == 0) {
-        sh.gave_up = 0; sh.bad = 0;
+        sh.gave_up = 0;
+        sh.a_mag = sh.b_mag = kNoMagnitudes;
         for (int i = 0; i < p.slots; ++i) { bar_init(smem_addr(&sh.b_full[i]), kProducers); bar_init(smem_addr(&sh.b_empty[i]), 1); }
         for (int i = 0; i < 2; ++i) {
             bar_init(smem_addr(&sh.d_full[i]), 1);
@@ -325,8 +338,6 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
         bar_init(smem_addr(&sh.drained), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (tid < kTensorMaxB) sh.b_max[tid] = 0;
-    if (tid >= 64 && tid < 64 + kTensorMaxStack) sh.a_max[tid - 64] = 0;
     // ---- result columns: 8-column groups of the nS Toeplitz matrices in turn
     for (int c = tid; c < D; c += kThreads) {
         const int blk = c >> 3, slot = blk % nS, b = slot / NR, n = blk / nS * 8 + (c & 7), sx = t.sx_lo + n;
@@ -345,13 +356,14 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
     tc_fence_after();
     const uint32_t tmem = sh.tmem;
 
-    // ---- largest magnitude of every B matrix of the block (the slice's rows)
-    for (int b = 0; b < t.nb; ++b) {
-        const unsigned* src = reinterpret_cast<const unsigned*>(t.b + ((size_t)b * H + t.y0) * W);
-        unsigned mx = 0;
-        for (int i = tid; i < rows * W; i += kThreads) mx = max(mx, __ldg(src + i) & 0x7fffffffu);
-        mx = __reduce_max_sync(0xffffffffu, mx);
-        if (lane == 0) atomicMax(&sh.b_max[b], mx);
+    // ---- magnitudes of the block's B matrices (the slice's rows)
+    {
+        Magnitudes m = kNoMagnitudes;
+        for (int b = 0; b < t.nb; ++b) {
+            const unsigned* src = reinterpret_cast<const unsigned*>(t.b + ((size_t)b * H + t.y0) * W);
+            for (int i = tid; i < rows * W; i += kThreads) see(m, __ldg(src + i));
+        }
+        merge(&sh.b_mag, m);
     }
 
     // ---- the lanes' output rows
@@ -409,13 +421,14 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
             const int kq = kc / 8, items = n_staged * p.J * kq;
             const uint32_t kq_rcp = (65536u + kq - 1) / kq;             // exact for the few thousand items there are
             const int first_row = t.row0 + t.y0;
+            Magnitudes mag = kNoMagnitudes;
             for (int i0 = 0; i0 < items; i0 += kThreads) {
                 const int i = min(i0 + tid, items - 1);                 // (the last items again rather than idle lanes)
                 const int r = (int)(((uint32_t)i * kq_rcp) >> 16), q = i - r * kq;
                 const int sr = r / p.J, j = r - sr * p.J;
                 int srow = first_row + sr;                              // (the stack starts over behind its end)
                 while (srow >= p.stack_rows) srow -= p.stack_rows;
-                const int g = srow / H, mat = g * p.J + j, local = (t.row0 % H + t.y0 + sr) / H * p.J + j;
+                const int g = srow / H, mat = g * p.J + j;
                 const bool there = mat < p.nA;
                 const float* src = t.a + ((size_t)(there ? mat : 0) * H + (srow - g * H)) * W;
                 const int u0 = p.Kp - 8 - (k0 + q * 8);                 // the item's columns: u0 + 7 down to u0
@@ -427,16 +440,15 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
 #pragma unroll
                     for (int k = 0; k < 8; ++k) v[k] = there && u0 + 7 - k < W ? __ldg(src + u0 + 7 - k) : 0.f;
                 }
-                unsigned mx = 0;
 #pragma unroll
-                for (int k = 0; k < 8; ++k) mx = max(mx, __float_as_uint(v[k]) & 0x7fffffffu);
-                if (there) atomicMax(&sh.a_max[local], mx);
+                for (int k = 0; k < 8; ++k) see(mag, __float_as_uint(v[k]));
                 uint4 part[3];
                 split8(v, part);
                 const uint32_t at = a_base + (uint32_t)(q * p.AR + ((sr % NR) * res_rows + sr / NR) * p.J + j) * 16;
 #pragma unroll
                 for (int s = 0; s < 3; ++s) sts128(at + s * a_part16 * 16, part[s]);
             }
+            merge(&sh.a_mag, mag);
             for (uint32_t i = tid * 16; i < p.slots * slot_bytes + 12 * ring_words; i += kThreads * 16) sts128(b_base + i, make_uint4(0, 0, 0, 0));
             if (tid == 0) {
                 int n = 0;
@@ -791,8 +803,6 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
     }
 
     // ---- operands the split does not cover: the block's results again, by the definition
-    if (tid < kTensorMaxStack && out_of_range(sh.a_max[tid])) sh.bad = 1;
-    if (tid < t.nb && out_of_range(sh.b_max[tid])) sh.bad = 1;
     __syncthreads();
     if (warp == kMmaWarp) {
         if (!ok) {
@@ -808,7 +818,7 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
         if (tid == 0) atomicAdd(&g_tensor_timeouts, 1u);
         return;
     }
-    if (sh.bad) {
+    if (out_of_range(sh.a_mag, sh.b_mag)) {
         direct_block(args, t);
         return;
     }
@@ -903,7 +913,6 @@ bool plan_tensor(const PairMap& pm, int H, int W, int sm_count, int max_slices, 
             p.AR = nR * p.res_rows * J | 1;
             // Toeplitz rows of a step, whatever the tile
             if (((W + 13) / 8 + 1) * nS * 8 > kTensorMaxItems) continue;
-            if (((128 / J * nR + 2 * H + rows) / H + 1) * J > kTensorMaxStack) continue;
             const int drain_warps = tensor_threads(D) / 32 - 4, NC = 4 * D / drain_warps;
             // (256 columns: one group of J lanes of a warp at most wraps at a time -- groups g and g' do together where
             // nR * (g - g') is a multiple of H)

@@ -173,6 +173,38 @@ def test_operands_outside_the_range_of_the_split(xc, oracle, shape, value):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("shape", [("n_to_m", 27, 43, 9, 35), ("n_to_mn", 48, 48, 16, 512), ("one_to_one", 225, 132, 1, 1)])
+@pytest.mark.parametrize("kind", ["far below the largest", "small products", "large"])
+def test_elements_and_products_at_the_ends_of_the_range(xc, oracle, shape, kind):
+    """Results that meet only elements below 2^-110 of matrices whose other elements are ordinary, results of matrices
+    whose products come near the smallest normal number, and elements up to 2^49 keep the precision of single-precision
+    sums: 0.2 sqrt(n) units of 2^-24 in the 2-norm for n products taken in sequence, and one for the margin."""
+    torch = pytest.importorskip("torch")
+    mode, rows, cols, nl, nr = shape
+    left, right = seeded_inputs(rows, cols, nl, nr, 17)
+    left, right = left + np.float32(0.5), right + np.float32(0.5)
+    if kind == "far below the largest":
+        left[:, rows - 1] *= np.float32(1e-35)                     # met alone by the first row of every right matrix
+    elif kind == "small products":
+        left, right = left * np.float32(2.0 ** -55), right * np.float32(2.0 ** -59)
+    else:
+        left, right = left * np.float32(2.0 ** 48), right * np.float32(2.0 ** 48)
+    got = run(xc, torch, shape, left, right).astype(np.float64)
+    assert xc.last_launch().startswith("kernel=tensor<"), xc.last_launch()
+    dl, dr = torch.from_numpy(left).cuda().double(), torch.from_numpy(right).cuda().double()
+    want = torch.empty(got.shape, dtype=torch.float64, device="cuda")
+    xc.run_device_f64(mode, dl.data_ptr(), dr.data_ptr(), want.data_ptr(), rows, cols, nl, nr, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    want = want.cpu().numpy()
+
+    def units(g, w, n):
+        return np.linalg.norm((g - w).ravel()) / np.linalg.norm(w.ravel()) * 2.0 ** 24 <= 1.0 + 0.2 * n ** 0.5
+
+    assert units(got, want, rows * cols)
+    assert units(got[:, -1], want[:, -1], cols)                    # shift rows - 1: one row of products
+
+
+@pytest.mark.gpu
 def test_side_stream_capture_and_missing_workspace(xc, oracle):
     torch = pytest.importorskip("torch")
     shape = ("one_to_one", 225, 132, 1, 1)

@@ -223,49 +223,122 @@ struct BlockTask {
     int y0, y1;
 };
 
-// The block's results by the definition, straight from global memory: operands that are out of the
-// split's range (see out_of_range).  Eight x shifts of one output row per thread.
-__device__ __noinline__ void direct_block(const TensorArgs& args, const BlockTask t) {
+// First element of the output row that stack row `srow`, matrix j of its group, belongs to before (0) or after (1) its
+// wrap; -1: no such matrix.
+__device__ __forceinline__ long long row_offset(const TensorPlan& p, const BlockTask& t, int srow, int j, int wrapped) {
+    const int H = p.H, OW = 2 * p.W - 1, OH = 2 * H - 1;
+    int g = srow / H;
+    const int sy = srow - g * H - (wrapped ? H : 0);
+    if (wrapped) g = (g + 1) * H < p.stack_rows ? g + 1 : 0;
+    const int a = g * p.J + j, at = (sy + H - 1) * OW;
+    if (srow >= p.stack_rows || a >= p.nA) return -1;
+    return (t.pair0 + (long long)a * p.stride_a) * ((long long)OH * OW) + (p.flip ? OH * OW - 1 - at : at);
+}
+
+// The block's results by the definition, in single precision FMAs: operands that the split does not cover.  Only
+// products that the definition has are formed (an infinity or NaN must not meet a zero that is none of the operand's).
+// A warp takes 32 stack rows, one per lane, and eight x shifts of one matrix B; the A rows stand in shared memory
+// as floats (as many columns at a time as fit: the results are then summed in the output), B's elements are the same
+// for all lanes.  Eight elements of either side are read for 64 FMAs.  One NaN in the left matrix of 64 x 64 1 x 512
+// costs 1140 us in all, where a kernel without reuse took 15.7 ms and the tile kernel takes 352 us.
+__device__ __noinline__ void direct_block(const TensorArgs& args, const BlockTask t, float* smem) {
     const TensorPlan& p = args.p;
-    const int H = p.H, W = p.W, OW = 2 * W - 1, OH = 2 * H - 1;
-    const int groups8 = p.DW / 8 * p.nB;
-    const int total = 128 * p.nR * 2 * groups8;
-    for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-        const int g8 = idx % groups8, row = idx / groups8;
-        const int srow = t.row0 + (row >> 1) / p.J, wrapped = row & 1;
-        const int b = g8 % p.nB, sx0 = t.sx_lo + g8 / p.nB * 8;
-        if (srow >= p.stack_rows || b >= t.nb || sx0 >= W) continue;
-        const int cy = srow % H;
-        int g = srow / H;
-        if (wrapped && (g + 1) * H >= p.stack_rows) g = -1;
-        const int a = (g + wrapped) * p.J + (row >> 1) % p.J;
-        if (a >= p.nA) continue;
-        const int ya = max(t.y0, wrapped ? H - cy : 0), yb = min(t.y1, wrapped ? H : H - cy);
-        if (ya >= yb) continue;
-        const int sy = wrapped ? cy - H : cy;
-        float sum[8];
+    const int H = p.H, W = p.W, OW = 2 * W - 1, OH = 2 * H - 1, J = p.J;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, warps = blockDim.x >> 5;
+    constexpr int kPitch = 9;                                         // of a warp's 32 x 8 results on their way out
+    float* turn = smem + warp * 32 * kPitch;
+    float* a_rows = smem + warps * 32 * kPitch;
+    const int rows = t.y1 - t.y0, lanes = 128 * p.nR, n_staged = lanes + (rows - 1) * J;
+    const int room = (int)((p.smem_bytes - (size_t)warps * 32 * kPitch * 4) / 4 / n_staged);
+    const int pitch = min((room - 1) | 1, W | 1), columns = min(pitch, W);      // odd: a column of rows meets all banks
+    const int row_groups = lanes / 32, units = row_groups * (p.DW / 8) * t.nb;
+    for (int ua = 0; ua < W; ua += columns) {
+        const int ub = min(W, ua + columns);
+        __syncthreads();
+        for (int i = tid; i < n_staged * (ub - ua); i += blockDim.x) {
+            const int q = i / (ub - ua), u = ua + i - q * (ub - ua), sr = q / J, mat_j = q - sr * J;
+            int srow = t.row0 + t.y0 + sr;
+            while (srow >= p.stack_rows) srow -= p.stack_rows;
+            const int g = srow / H, mat = g * J + mat_j;
+            a_rows[q * pitch + u - ua] = mat < p.nA ? __ldg(t.a + ((size_t)mat * H + (srow - g * H)) * W + u) : 0.f;
+        }
+        __syncthreads();
+        for (int unit = warp; unit < units; unit += warps) {
+            const int c8 = unit / row_groups, i = (unit - c8 * row_groups) * 32 + lane, b = c8 % t.nb, sx0 = t.sx_lo + c8 / t.nb * 8;
+            const int srow = t.row0 + i / J, wrap = H - srow % H;              // the row y with which this lane runs on into the next matrix
+            const long long off0 = row_offset(p, t, srow, i % J, 0), off1 = row_offset(p, t, srow, i % J, 1);
+            const int x_lo = max(0, ua - sx0 - 7), x_hi = min(W, ub - sx0);    // columns of B that meet the chunk at any of the shifts
+            if (sx0 >= W || (x_hi <= x_lo && ua > 0)) continue;
+            float acc[8];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) sum[j] = 0.f;
-        for (int y = ya; y < yb; ++y) {
-            const float* ar = t.a + ((size_t)a * H + (y + sy)) * W;
-            const float* br = t.b + ((size_t)b * H + y) * W;
-            for (int u = max(0, sx0); u < min(W, W + sx0 + 7); ++u) {
-                const float av = __ldg(ar + u);
+            for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+            // the sums of the lanes in `who` are result rows: through shared memory, so that eight neighbours leave together
+            const auto put = [&](unsigned who, long long off) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int x = u - sx0 - j;
-                    if (x >= 0 && x < W) sum[j] = fmaf(av, __ldg(br + x), sum[j]);
+                for (int j = 0; j < 8; ++j) turn[lane * kPitch + j] = acc[j];
+                __syncwarp();
+                const int sx = sx0 + (lane & 7), col = p.flip ? -(sx + W - 1) : sx + W - 1;
+                while (who) {
+                    int src = -1;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {                              // a lane of `who` for every eight lanes
+                        if (who && lane >> 3 == k) src = __ffs(who) - 1;
+                        who &= who - 1;
+                    }
+                    const long long to = __shfl_sync(0xffffffffu, off, max(src, 0));
+                    if (src >= 0 && to >= 0 && sx < W) {
+                        float* o = t.out + to + b * (p.stride_b * ((long long)OH * OW)) + col;
+                        const float v = turn[src * kPitch + (lane & 7)];
+                        *o = ua > 0 ? *o + v : v;
+                    }
+                }
+                __syncwarp();
+            };
+            const float* br = t.b + ((size_t)b * H + t.y0) * W;
+            const float* ar = a_rows + i * pitch + sx0 - ua;                   // column x of B meets ar[x + j] at shift sx0 + j
+            for (int y = t.y0; y < t.y1; ++y, br += W, ar += J * pitch) {
+                const unsigned who = __ballot_sync(0xffffffffu, y == wrap && y > t.y0);
+                if (who) {
+                    put(who, off0);
+                    if (y == wrap) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+                    }
+                }
+                float w[15];
+                {
+                    const int lo = ua - sx0 - x_lo, hi = ub - sx0 - x_lo;
+#pragma unroll
+                    for (int k = 0; k < 7; ++k) w[k + 8] = k >= lo && k < hi ? ar[x_lo + k] : 0.f;
+                }
+#pragma unroll 1
+                for (int x = x_lo; x < x_hi; x += 8) {
+                    const int lo = ua - sx0 - x, hi = ub - sx0 - x;            // elements of the window that are columns of the chunk
+#pragma unroll
+                    for (int k = 0; k < 7; ++k) w[k] = w[k + 8];
+                    if (lo <= 0 && hi >= 15 && x + 8 <= W) {
+                        float v[8];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) { w[k + 7] = ar[x + 7 + k]; v[k] = __ldg(br + x + k); }
+#pragma unroll
+                        for (int k = 0; k < 8; ++k)
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) acc[j] = fmaf(w[k + j], v[k], acc[j]);
+                    } else {
+#pragma unroll
+                        for (int k = 7; k < 15; ++k) w[k] = k >= lo && k < hi ? ar[x + k] : 0.f;
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            if (x + k >= W) break;
+                            const float v = __ldg(br + x + k);
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                if (k + j >= lo && k + j < hi) acc[j] = fmaf(w[k + j], v, acc[j]);
+                        }
+                    }
                 }
             }
-        }
-        const long long pair = t.pair0 + (long long)a * p.stride_a + (long long)b * p.stride_b;
-        float* o = t.out + pair * ((long long)OH * OW);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int sx = sx0 + j;
-            if (sx >= W) continue;
-            const int at = (sy + H - 1) * OW + sx + W - 1;
-            o[p.flip ? OH * OW - 1 - at : at] = sum[j];
+            put(0xffffffffu, wrap < t.y1 ? off1 : off0);
         }
     }
 }
@@ -368,16 +441,6 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
 
     // ---- the lanes' output rows
     const int half_col = (warp >> 2) * NC;
-    // first element of the output row of matrix j of a stack row's group, for its shift before (0) or after (1)
-    // the wrap; -1: no such matrix
-    auto row_offset = [&](int srow, int j, int wrapped) -> long long {
-        int g = srow / H;
-        const int sy = srow - g * H - (wrapped ? H : 0);
-        if (wrapped) g = (g + 1) * H < p.stack_rows ? g + 1 : 0;
-        const int a = g * p.J + j, at = (sy + H - 1) * OW;
-        if (srow >= p.stack_rows || a >= p.nA) return -1;
-        return (t.pair0 + (long long)a * p.stride_a) * ((long long)OH * OW) + (p.flip ? OH * OW - 1 - at : at);
-    };
     bool wrapped[NR];                              // the sums at hand belong to the shift after the wrap
     int wrap_step[NR];                             // step with which a drain lane's rows run on into the next group; -1: never
 #pragma unroll
@@ -385,8 +448,8 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
         const int m = (warp & 3) * 32 + lane, srow = t.row0 + m / p.J * NR + rho, y = H - srow % H;
         wrap_step[rho] = srow < p.stack_rows && y > t.y0 && y < t.y1 ? y - t.y0 + rho : -1;
         if (warp < 4) {
-            sh.row_out[0][rho][m] = row_offset(srow, m % p.J, 0);
-            sh.row_out[1][rho][m] = row_offset(srow, m % p.J, 1);
+            sh.row_out[0][rho][m] = row_offset(p, t, srow, m % p.J, 0);
+            sh.row_out[1][rho][m] = row_offset(p, t, srow, m % p.J, 1);
         }
         wrapped[rho] = y <= t.y0;
     }
@@ -403,7 +466,7 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
         for (int c = 0; c < NC; ++c) { sum[c] = 0.f; if (!kResident) rest[c] = 0.f; }
     };
     if (MANY) no_sums();
-    bool ok = true;
+    bool ok = true, covered = true;
     for (int k0 = 0; k0 < p.Kp; k0 += p.KC) {
         const int kc = min(p.KC, p.Kp - k0);
         const int X0 = p.Kp - 1 - t.sx_lo - k0;    // column of B that chunk column k meets at result column n: X0 - n - k
@@ -470,6 +533,8 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
             }
             fence_async();
             __syncthreads();
+            // (what the split does not cover is not worth its products: the same for every thread)
+            if (out_of_range(sh.a_mag, sh.b_mag)) { covered = false; break; }
         }
 
         const int back = MANY ? pass & 1 : 0;
@@ -755,7 +820,7 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
 
     // ---- the walk's end: all sums are result rows.  Through shared memory (the A side is done with: all
     // products have completed), 16 lanes at a time, so that a store instruction writes up to 32 neighbours.
-    if (ok && warp < kDrainWarps) {
+    if (ok && covered && warp < kDrainWarps) {
         float* tile = reinterpret_cast<float*>(smem) + warp * 16 * (NC + 1);
         if (kResident) {
             const uint32_t t_addr = tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)half_col + D;
@@ -818,8 +883,8 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
         if (tid == 0) atomicAdd(&g_tensor_timeouts, 1u);
         return;
     }
-    if (out_of_range(sh.a_mag, sh.b_mag)) {
-        direct_block(args, t);
+    if (!covered) {
+        direct_block(args, t, reinterpret_cast<float*>(smem));
         return;
     }
     // ---- the corners of a result are single products: rounded once, as the definition has them (the three

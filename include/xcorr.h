@@ -403,19 +403,20 @@ XCORR_API void xcorr_reset_launch_count(void);
 /* Health of the current device as this library sees it: synchronises the device, then returns
  * XCORR_ERR_CUDA if an earlier launch failed, XCORR_ERR_TIMEOUT if a bounded device-side wait of
  * the library's kernels gave up since the last call of this function (the blocks concerned
- * dropped their work and returned, so results of launches since then are incomplete; the count
- * is in xcorr_last_error_string() and is cleared by this call, the context stays usable), else
+ * dropped their work and returned, so results of launches since then are incomplete; the counts
+ * are in xcorr_last_error_string() and are cleared by this call, the context stays usable), else
  * XCORR_OK.  Stands in for the CUCH(cudaDeviceSynchronize()); CUCH(cudaGetLastError()) pair of
  * main.cpp:267-270. */
 XCORR_API xcorr_status xcorr_check_device(void);
 
-/* Test hook for the one device-side wait of the library (a block of the tile kernel waiting for
- * its bulk copies into shared memory).  poll_limit > 0 replaces the number of polls after which
- * the wait gives up (default about 4 million); surplus_bytes > 0 makes every block announce that
- * many bytes more than its copies deliver, so the wait cannot succeed and runs out: the launch
- * then reports XCORR_ERR_TIMEOUT through xcorr_check_device without any fault, hang or lost
- * context (the block takes the surplus back and lets its real copies land before it returns).
- * (0, 0) restores normal operation.  Process-wide; affects launches made after the call. */
+/* Test hook for the device-side waits of the library, all within a block: of the tile kernel for
+ * its bulk copies into shared memory, and between the roles of the tensor kernel.  poll_limit > 0
+ * replaces the number of polls after which a wait gives up (default about 4 million);
+ * surplus_bytes > 0 makes every block of the tile kernel announce that many bytes more than its
+ * copies deliver, and every block of the tensor kernel expect an arrival more than its products
+ * give, so that the wait cannot succeed and runs out: the launch then reports XCORR_ERR_TIMEOUT
+ * through xcorr_check_device without any fault, hang or lost context (the block lets its copies
+ * and products land before it returns).  (0, 0) restores normal operation.  Process-wide; affects launches made after the call. */
 XCORR_API void xcorr_debug_stage_wait(uint32_t poll_limit, uint32_t surplus_bytes);
 
 /* Measured FP32 FFMA throughput of the current device in FLOP/s: a dependency-free

@@ -85,7 +85,7 @@ struct DeviceGuard {
     DeviceGuard& operator=(const DeviceGuard&) = delete;
 };
 
-// xcorr_debug_stage_wait: bound and surplus of the tile kernel's staging wait (test hook).
+// xcorr_debug_stage_wait: bound and surplus of the device-side waits (test hook).
 std::atomic<unsigned> g_stage_wait_limit{kStageWaitLimit};
 std::atomic<unsigned> g_stage_expect_surplus{0};
 
@@ -877,6 +877,8 @@ xcorr_status run_device(int32_t mode, const float* d_left, const float* d_right,
         ta.out = tp.S > 1 ? static_cast<float*>(d_ws) : d_out;
         ta.slice_floats = total_out;
         ta.p = tp;
+        ta.wait_limit = g_stage_wait_limit.load(std::memory_order_relaxed);
+        ta.withheld = g_stage_expect_surplus.load(std::memory_order_relaxed) ? 1 : 0;
         t_note.kind = LaunchNote::kTensor; t_note.tensor = tp;
         XC_CUDA(launch_tensor(ta, device, stream));
         ++t_launch_count;
@@ -1309,12 +1311,10 @@ xcorr_status xcorr_check_device(void) {
         XC_CUDA(tile_stage_timeouts(&timeouts));
         unsigned tensor_timeouts = 0;
         XC_CUDA(tensor_wait_timeouts(&tensor_timeouts));
-        if (tensor_timeouts != 0)
-            return fail(XCORR_ERR_TIMEOUT, std::to_string(tensor_timeouts) + " block(s) of tensor_kernel gave up a bounded wait "
-                        "and dropped their work; results of the launches since the last check are incomplete");
-        if (timeouts != 0)
-            return fail(XCORR_ERR_TIMEOUT, std::to_string(timeouts) + " block(s) of tile_kernel gave up a bounded staging wait "
-                        "and dropped their work; results of the launches since the last check are incomplete");
+        if (tensor_timeouts != 0 || timeouts != 0)
+            return fail(XCORR_ERR_TIMEOUT, std::to_string(timeouts) + " block(s) of tile_kernel and " + std::to_string(tensor_timeouts) +
+                        " block(s) of tensor_kernel gave up a bounded wait and dropped their work; results of the launches since "
+                        "the last check are incomplete");
         return XCORR_OK;
     });
 }

@@ -168,6 +168,8 @@ struct TensorArgs {
     float* out;        // the results, or the first partial image
     int vec_ok;        // A rows may be fetched with 16-byte loads
     unsigned long long slice_floats;     // floats between partial images
+    unsigned wait_limit;                 // polls after which a wait gives up
+    unsigned withheld;                   // test hook: arrivals the result barriers expect and never get
     TensorPlan p;
 };
 

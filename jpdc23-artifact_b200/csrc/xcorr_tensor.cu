@@ -110,9 +110,9 @@ __device__ __forceinline__ bool bar_poll(uint32_t bar, uint32_t parity) {
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
-// Bounded: false after kStageWaitLimit polls, or once another warp of the block has given up.
-__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* gave_up) {
-    for (unsigned it = 0; it < kStageWaitLimit; ++it) {
+// Bounded: false after `limit` polls, or once another warp of the block has given up.
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* gave_up, unsigned limit) {
+    for (unsigned it = 0; it < limit; ++it) {
         if (bar_poll(bar, parity)) return true;
         if ((it & 63) == 63 && *gave_up) return false;
     }
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
         sh.a_mag = sh.b_mag = kNoMagnitudes;
         for (int i = 0; i < p.slots; ++i) { bar_init(smem_addr(&sh.b_full[i]), kProducers); bar_init(smem_addr(&sh.b_empty[i]), 1); }
         for (int i = 0; i < 2; ++i) {
-            bar_init(smem_addr(&sh.d_full[i]), 1);
+            bar_init(smem_addr(&sh.d_full[i]), 1 + args.withheld);
             bar_init(smem_addr(&sh.d_empty[i]), kDrainWarps);
             bar_init(smem_addr(&sh.rest_free[i]), kDrainWarps);
         }
@@ -595,7 +595,7 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
                     if (i + 1 < steps_y) wrap_at(i + 1); else who0 = who1 = 0;
                     if (!(who0 | who1) && lane == 0) bar_arrive(smem_addr(&sh.rest_free[it & 1]));
                 }
-                ok = bar_wait(smem_addr(&sh.d_full[buffer]), (kResident ? it : it >> 1) & 1, &sh.gave_up);
+                ok = bar_wait(smem_addr(&sh.d_full[buffer]), (kResident ? it : it >> 1) & 1, &sh.gave_up, args.wait_limit);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
@@ -712,7 +712,7 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
                     if (i + 1 < rows) ahead[j] = __ldg(from[j] + (back ? -(long long)(i + 1) * W : (long long)(i + 1) * W));
                 }
                 asm volatile("bar.sync 1, %0;" :: "n"(kProducers) : "memory");
-                if (ok && use > 0) ok = bar_wait(smem_addr(&sh.b_empty[slot]), (use - 1) & 1, &sh.gave_up);
+                if (ok && use > 0) ok = bar_wait(smem_addr(&sh.b_empty[slot]), (use - 1) & 1, &sh.gave_up, args.wait_limit);
                 ok = __all_sync(0xffffffffu, ok);
                 const uint32_t dst0 = b_base + slot * slot_bytes, set_bytes = (uint32_t)p.nB * row_bytes;
                 const uint32_t src0 = ring_base + (uint32_t)(place & (kRowRing - 1)) * set_bytes;
@@ -754,9 +754,9 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
             for (int i = 0; ok && i < steps_y; ++i) {
                 const unsigned it = it_base + i, use = it / p.slots;
                 const int slot = (int)(it - use * p.slots);
-                ok = bar_wait(smem_addr(&sh.b_full[slot]), use & 1, &sh.gave_up);
-                if (kResident && ok && it >= 1) ok = bar_wait(smem_addr(&sh.rest_free[(it - 1) & 1]), ((it - 1) >> 1) & 1, &sh.gave_up);
-                if (!kResident && ok && it >= 2) ok = bar_wait(smem_addr(&sh.d_empty[it & 1]), ((it >> 1) - 1) & 1, &sh.gave_up);
+                ok = bar_wait(smem_addr(&sh.b_full[slot]), use & 1, &sh.gave_up, args.wait_limit);
+                if (kResident && ok && it >= 1) ok = bar_wait(smem_addr(&sh.rest_free[(it - 1) & 1]), ((it - 1) >> 1) & 1, &sh.gave_up, args.wait_limit);
+                if (!kResident && ok && it >= 2) ok = bar_wait(smem_addr(&sh.d_empty[it & 1]), ((it >> 1) - 1) & 1, &sh.gave_up, args.wait_limit);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 tc_fence_after();
@@ -789,7 +789,7 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
                 __syncwarp();
                 if (kResident) {
                     // the large products last: their sums of the row before are drained meanwhile
-                    if (it >= 1) ok = bar_wait(smem_addr(&sh.d_empty[0]), (it - 1) & 1, &sh.gave_up);
+                    if (it >= 1) ok = bar_wait(smem_addr(&sh.d_empty[0]), (it - 1) & 1, &sh.gave_up, args.wait_limit);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     tc_fence_after();
@@ -871,7 +871,7 @@ __global__ void __launch_bounds__(kTensorThreads<D>, 1) tensor_kernel(const __gr
     __syncthreads();
     if (warp == kMmaWarp) {
         if (!ok) {
-            // products may be in flight: let them land before their memory goes
+            // products may be in flight: let them land before their memory goes (with the full limit, whatever the others had)
             if (elect_one()) tc_commit(smem_addr(&sh.drained));
             __syncwarp();
             for (unsigned it = 0; it < kStageWaitLimit && !bar_poll(smem_addr(&sh.drained), 0); ++it) {}

@@ -784,9 +784,9 @@ def test_staged_and_split_hints_are_checked(xc):
 
 
 def test_bounded_staging_wait_gives_up_and_reports(xc, oracle):
-    """The one device-side wait of the library (a block waiting for its bulk copies) is bounded.
-    The test hook announces 64 bytes more than the copies deliver and lowers the poll limit, so
-    the wait runs out: no fault, no hang -- the blocks drop their work, the launch is reported as
+    """The tile kernel's wait (a block waiting for its bulk copies) is bounded.  The test hook
+    announces 64 bytes more than the copies deliver and lowers the poll limit, so the wait runs
+    out: no fault, no hang -- the blocks drop their work, the launch is reported as
     XCORR_ERR_TIMEOUT by the device check (once), and the next launch is right again."""
     lib = xc.lib()
     xc.check_device()

@@ -270,3 +270,38 @@ def test_side_stream_capture_and_missing_workspace(xc, oracle):
     assert xc.last_launch().startswith("kernel=tensor<")
     got = out[1:].cpu().numpy().reshape(want.shape)
     assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("polls", [1, 4096])
+def test_waits_that_run_out_are_reported(xc, oracle, polls):
+    """The waits between the kernel's roles are bounded.  The test hook keeps one arrival from the barrier that says a
+    row's products are done, and lowers the limit: at one poll the first wait of any role gives up, at 4096 the
+    products of two rows are issued before the warps that wait for them do.  No fault, no hang: the blocks drop their work,
+    the check reports them once and beside those of the tile kernel, and the next launch is right."""
+    torch = pytest.importorskip("torch")
+    lib = xc.lib()
+    xc.check_device()
+    # several matrices B, one chunk of columns; one pair in row slices, several chunks
+    shapes = [("n_to_m", 27, 43, 9, 35), ("one_to_one", 225, 132, 1, 1)]
+    inputs = [seeded_inputs(*s[1:], 5) for s in shapes]
+    small = seeded_inputs(32, 32, 1, 6, 77)
+    for tile_too in (False, True):
+        lib.xcorr_debug_stage_wait(polls, 64)
+        try:
+            for s, (left, right) in zip(shapes, inputs):
+                run(xc, torch, s, left, right)
+                assert xc.last_launch().startswith("kernel=tensor<")
+            if tile_too:
+                run(xc, torch, ("one_to_many", 32, 32, 1, 6), *small, xc.make_hints(kernel="tile"))
+            assert lib.xcorr_check_device() == 8
+            text = lib.xcorr_last_error_string().decode()
+            assert "gave up" in text and " 0 block(s) of tensor_kernel" not in text
+            assert text.startswith("0 block(s) of tile_kernel") != tile_too
+        finally:
+            lib.xcorr_debug_stage_wait(0, 0)
+        xc.check_device()                                      # both counts were cleared by the report
+        for s, (left, right) in zip(shapes, inputs):
+            got, want = run(xc, torch, s, left, right), reference(oracle, s, left, right)
+            assert np.abs(got - want).max() <= 1e-5 * np.abs(want).max()
+    xc.check_device()

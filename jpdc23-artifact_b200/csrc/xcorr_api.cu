@@ -1286,14 +1286,16 @@ xcorr_status xcorr_fft_f32(int32_t mode, const float* d_left, const float* d_rig
         int device = 0;
         if ((st = current_device_info(&dev, &device)) != XCORR_OK) return st;
         std::string err;
-        int launches = 0;
+        FftRoute route{};
         const int rc = fft_run(d_left, d_right, d_out, (int)rows, (int)cols, pm, n_right, layout == XCORR_FFT_RAW,
-                               d_workspace, device, dev.sm_count, static_cast<cudaStream_t>(stream), &err, &launches);
-        t_launch_count += (uint64_t)launches;
+                               d_workspace, device, dev.sm_count, static_cast<cudaStream_t>(stream), &err, &route);
+        t_launch_count += (uint64_t)route.launches;
         if (rc != 0) return fail(XCORR_ERR_CUDA, err);
         char buf[256];
-        std::snprintf(buf, sizeof buf, "kernel=fft transform=%ux%u inputs=%llu pairs=%llu product=%s layout=%s workspace=%zu",
-                      2 * rows, 2 * cols, (unsigned long long)pm.n_left + n_right, (unsigned long long)pm.n_left * pm.m,
+        std::snprintf(buf, sizeof buf, "kernel=fft route=%s transform=%dx%d inputs=%llu pairs=%llu product=%s layout=%s workspace=%zu",
+                      route.block ? "block" : "cufft", route.rows, route.cols, (unsigned long long)pm.n_left + n_right,
+                      (unsigned long long)pm.n_left * pm.m,
+                      route.block ? (route.rights_once ? "in-block right-spectra=once" : "in-block right-spectra=per-pair") :
                       lay.product_in_place ? "in-place" : "separate", layout == XCORR_FFT_RAW ? "raw" : "normalized",
                       lay.total);
         set_launch_text(buf);

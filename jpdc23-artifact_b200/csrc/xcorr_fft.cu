@@ -222,7 +222,8 @@ FftLayout fft_workspace_layout(const PairMap& pm, int H, int W, unsigned n_right
 
 int fft_run(const float* left, const float* right, float* out, int H, int W, const PairMap& pm, unsigned n_right,
             int raw_result, void* workspace, int device, int sm_count, cudaStream_t stream, std::string* err,
-            int* launches) {
+            FftRoute* route) {
+    *route = FftRoute{0, 2 * H, 2 * W, 1, 0};
     const FftLayout lay = fft_workspace_layout(pm, H, W, n_right, raw_result);
     char* ws = static_cast<char*>(workspace);
     float* padded = reinterpret_cast<float*>(ws + lay.padded_off);
@@ -243,7 +244,7 @@ int fft_run(const float* left, const float* right, float* out, int H, int W, con
 
     // small enough for one SM: one block per pair does it all
     cudaError_t block_err = cudaSuccess;
-    if (!raw_result && fft_block_run(left, right, out, H, W, pm, n_right, workspace, lay.total, device, sm_count, stream, &block_err, launches))
+    if (!raw_result && fft_block_run(left, right, out, H, W, pm, n_right, workspace, lay.total, device, sm_count, stream, &block_err, route))
         return cuda_check(block_err, "fft_block_kernel") ? 1 : 0;
 
     // 1. pad both inputs: left matrices first, right matrices after them
@@ -259,7 +260,7 @@ int fft_run(const float* left, const float* right, float* out, int H, int W, con
         else     fft_pad_kernel<false><<<grid, kThreads, 0, stream>>>(src, dst, H, W, rows_total);
         if (cuda_check(cudaGetLastError(), "fft_pad_kernel")) return 1;
     }
-    *launches += 2;
+    route->launches += 2;
 
     {
         // 2. forward transforms of all inputs in one batch; 4. inverse transforms of all pairs
@@ -283,7 +284,7 @@ int fft_run(const float* left, const float* right, float* out, int H, int W, con
         r = cufftExecC2R(inv, reinterpret_cast<cufftComplex*>(product), raw);
         if (r != CUFFT_SUCCESS) { *err = std::string("cuFFT inverse: ") + cufft_name(r); return 2; }
     }
-    *launches += 1;
+    route->launches += 1;
 
     // 5. unpack to the direct path's layout
     if (!raw_result) {
@@ -291,7 +292,7 @@ int fft_run(const float* left, const float* right, float* out, int H, int W, con
         fft_unpack_kernel<<<grid_for(rows_total * 32, sm_count), kThreads, 0, stream>>>(
             raw, out, H, W, 1.0f / (4.0f * (float)H * (float)W), rows_total);
         if (cuda_check(cudaGetLastError(), "fft_unpack_kernel")) return 1;
-        *launches += 1;
+        route->launches += 1;
     }
     return 0;
 }

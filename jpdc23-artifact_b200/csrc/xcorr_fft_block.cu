@@ -415,7 +415,7 @@ cudaError_t launch(const FftBlockArgs& a, unsigned grid, size_t bytes, int devic
 }  // namespace
 
 bool fft_block_run(const float* left, const float* right, float* out, int H, int W, const PairMap& pm, unsigned n_right,
-                   void* workspace, size_t workspace_bytes, int device, int sm_count, cudaStream_t stream, cudaError_t* err, int* launches) {
+                   void* workspace, size_t workspace_bytes, int device, int sm_count, cudaStream_t stream, cudaError_t* err, FftRoute* route) {
     FftBlockArgs a{};
     size_t bytes = 0;
     for (int small = 0; small < 2; ++small) {
@@ -438,9 +438,10 @@ bool fft_block_run(const float* left, const float* right, float* out, int H, int
     const bool shared_rights = pm.n_left > 1 && pm.right_stride == 0 && pairs > wave;
     const size_t spectra = pm.n_left + (shared_rights ? (size_t)n_right : 0);
     if (spectra * spectrum * sizeof(float2) > workspace_bytes || pairs > 0x7fffffffull || n_right > 0x7fffffffu) return false;
+    *route = FftRoute{1, a.cols.n, a.rows.n, shared_rights ? 1 : 0, 0};
     float2* store = static_cast<float2*>(workspace);
     const auto run = [&](bool pair, unsigned grid) -> cudaError_t {
-        ++*launches;
+        ++route->launches;
         // three blocks of 256 threads per SM where they fit, two of 384, else one of 512; no more blocks than SMs:
         // 512 threads, the time is one block's (one 60 x 60 pair 29 -> 26 us, 64 x 64 9 x 14 43 -> 27 us with the
         // launch saved below; the left spectra of 64 x 64 1 x 512, one block before all others, 62 -> 60 us)

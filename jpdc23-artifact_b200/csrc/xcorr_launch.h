@@ -64,15 +64,17 @@ struct FftLayout {
 };
 FftLayout fft_workspace_layout(const PairMap& pm, int H, int W, unsigned n_right, int raw_result);
 // Enqueues the whole path on `stream`.  0 = ok, 1 = CUDA error, 2 = cuFFT error (*err says which);
-// *launches is increased by the number of own kernels launched.
+// *route: what ran -- one block per pair (transforms of rows x cols points, the right spectra made once or by every
+// pair) or cuFFT's batches -- and the number of own kernels launched.
+struct FftRoute { int block, rows, cols, rights_once, launches; };
 int fft_run(const float* left, const float* right, float* out, int H, int W, const PairMap& pm, unsigned n_right,
             int raw_result, void* workspace, int device, int sm_count, cudaStream_t stream, std::string* err,
-            int* launches);
+            FftRoute* route);
 // The normalized layout in one block per pair, for sizes whose half spectrum fits one SM (xcorr_fft_block.cu).
 // false: not such a size (nothing was launched); true: *err is the launches' status.
 bool fft_block_run(const float* left, const float* right, float* out, int H, int W, const PairMap& pm, unsigned n_right,
                    void* workspace, size_t workspace_bytes, int device, int sm_count, cudaStream_t stream, cudaError_t* err,
-                   int* launches);
+                   FftRoute* route);
 void fft_release_plans();
 
 }  // namespace xcorr

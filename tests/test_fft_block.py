@@ -1,6 +1,8 @@
 """The FFT path's one-block kernel (csrc/xcorr_fft_block.cu) at every kind of transform length it uses --
 each radix as a first, inner and last pass, single passes, odd and even matrix heights -- and on both sides of
 the rules that choose it, against double-precision transforms."""
+import re
+
 import numpy as np
 import pytest
 
@@ -32,6 +34,16 @@ def check(xc, mode, rows, cols, nl, nr, launches=None):
     assert bool((ws[:guard] == 77).all()) and bool((ws[guard + wsb:] == 77).all())
     if launches is not None:
         assert xc.launch_count() == launches
+    # the text names what ran: lengths that hold the result, a power of two times at most one 3 and one 5, or cuFFT's
+    text = xc.last_launch()
+    p, q = (int(v) for v in re.search(r" transform=(\d+)x(\d+) ", text).groups())
+    if " route=block " in text:
+        assert "product=in-block" in text and ("right-spectra=once" in text) == (xc.launch_count() == 3)
+        for length, need in ((p, 2 * rows - 1), (q, 2 * cols - 1)):
+            odd = length // (length & -length)
+            assert length >= need and length % 2 == 0 and odd in (1, 3, 5, 15)
+    else:
+        assert " route=cufft " in text and (p, q) == (2 * rows, 2 * cols) and xc.launch_count() == 4
     p = (2 * rows, 2 * cols)
     fl, fr = torch.fft.rfft2(left.double(), s=p), torch.fft.rfft2(right.double(), s=p).conj()
     f = (fl[:, None] * fr[None]).reshape(-1, *fl.shape[1:]) if mode == "n_to_m" else fl.repeat_interleave(nr // nl, 0) * fr

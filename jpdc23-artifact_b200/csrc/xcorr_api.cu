@@ -877,6 +877,7 @@ xcorr_status run_device(int32_t mode, const float* d_left, const float* d_right,
         ta.out = tp.S > 1 ? static_cast<float*>(d_ws) : d_out;
         ta.slice_floats = total_out;
         ta.p = tp;
+        ta.vec_ok = W % 4 == 0 && reinterpret_cast<uintptr_t>(ta.a) % 16 == 0;
         ta.wait_limit = g_stage_wait_limit.load(std::memory_order_relaxed);
         ta.withheld = g_stage_expect_surplus.load(std::memory_order_relaxed) ? 1 : 0;
         t_note.kind = LaunchNote::kTensor; t_note.tensor = tp;

@@ -273,6 +273,29 @@ def test_side_stream_capture_and_missing_workspace(xc, oracle):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("offset", [0, 1, 4])
+@pytest.mark.parametrize("shape", [("n_to_m", 20, 48, 33, 63), ("n_to_m", 20, 64, 35, 31), ("one_to_one", 225, 132, 1, 1)])
+def test_operands_at_any_alignment(xc, oracle, shape, offset):
+    """A rows are staged with 16-byte loads where the operand and its rows allow it: operands 0, 4 and 16 bytes into a
+    buffer, odd numbers of matrices interleaved by two (the absent one is staged as zeros)."""
+    torch = pytest.importorskip("torch")
+    mode, rows, cols, nl, nr = shape
+    left, right = seeded_inputs(rows, cols, nl, nr, 6)
+    want = reference(oracle, shape, left, right)
+    pad = np.full(offset, 1e30, np.float32)
+    dl = torch.from_numpy(np.concatenate([pad, left.ravel()])).cuda()
+    dr = torch.from_numpy(np.concatenate([pad, right.ravel()])).cuda()
+    out = torch.full((int(np.prod(xc.out_shape(*shape))),), float("nan"), dtype=torch.float32, device="cuda")
+    wsb = xc.workspace_bytes(*shape)
+    ws = torch.empty(wsb + 16, dtype=torch.uint8, device="cuda")
+    xc.run_device(mode, dl.data_ptr() + 4 * offset, dr.data_ptr() + 4 * offset, out.data_ptr(), rows, cols, nl, nr, None,
+                  ws.data_ptr() if wsb else 0, wsb, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert xc.last_launch().startswith("kernel=tensor<"), xc.last_launch()
+    assert np.abs(out.cpu().numpy().reshape(want.shape) - want).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("polls", [1, 4096])
 def test_waits_that_run_out_are_reported(xc, oracle, polls):
     """The waits between the kernel's roles are bounded.  The test hook keeps one arrival from the barrier that says a

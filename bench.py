@@ -961,7 +961,9 @@ def main():
                 if len(parts) == 3 and parts[0] == dom:
                     if parts[2].strip() == plan_signature(plans[dom]):
                         traffic = int(parts[1])
-                        traffic_note = "ncu capture profiles/tile_kernel_%s.md, plan %s" % (dom, parts[2].strip())
+                        traffic_note = "ncu capture profiles/%s.md, plan %s" % (
+                            "tensor_kernel_and_fft_block" if parts[2].startswith("tensor") else "tile_kernel_" + dom, parts[2].strip())
+                        break                                 # (a configuration has a line per plan captured)
                     else:
                         traffic_note = ("the capture on file is for plan %s, this run used %s: figure withheld"
                                         % (parts[2].strip(), plan_signature(plans[dom])))

@@ -74,14 +74,19 @@ typedef enum xcorr_kernel {
     XCORR_KERNEL_AUTO = 0,          /* per-shape selection: the tile kernel, for a handful of small overlaps the
                                        warp-per-overlap kernel, and from some tens of microseconds of work on the
                                        tensor cores (each float as three bfloat16 parts, sums in 32 bits; bit-identical
-                                       from run to run) where those are estimated faster and no less precise.  A
-                                       result may differ from the tile kernel's in its last bits */
+                                       from run to run) where those are estimated faster and no less precise in the
+                                       2-norm.  A result may differ from the tile kernel's in its last bits; those of
+                                       the tensor cores come out smaller in the mean, by up to about one unit of
+                                       2^-24 for large overlaps, where the tile kernel's errors are larger but have no
+                                       sign.  Infinities, NaN, magnitudes of 2^50 and more or of less than 2^-110, and
+                                       products below 2^-100 are left to FMAs within the same launch (1.3 to
+                                       4.7 times the tile kernel's time) */
     XCORR_KERNEL_TILE = 1,          /* register-tiled circular-class kernel (the fast path) */
     XCORR_KERNEL_OVERLAP_WISE = 2,  /* one thread per overlap -- run_cross_corr_naive_original, naive_original.cu:131-161 */
     XCORR_KERNEL_WARP_PER_OVERLAP = 3, /* one warp per overlap -- run_ccn_warp_per_shift, naive_warp_per_shift.cu:308-335.
                                        The automatic choice for a handful of small overlaps (at most 8000 in the
                                        call, rows and columns up to 32: a 16 x 16 or 32 x 32 pair) */
-    XCORR_KERNEL_FFT = 4,           /* the cuFFT path (xcorr_fft_f32 with the normalized layout); needs the
+    XCORR_KERNEL_FFT = 4,           /* the FFT path (xcorr_fft_f32 with the normalized layout); needs the
                                        workspace xcorr_workspace_bytes() reports for this hint.  Never chosen
                                        automatically: its rounding differs from the direct path's */
     XCORR_KERNEL_WARP_STAGED = 5    /* one warp per overlap, operands staged through shared memory --
@@ -207,8 +212,8 @@ XCORR_API xcorr_status xcorr_n_to_m_f32(const float* d_left, const float* d_righ
  * allocation after start-up, a process whose memory pool is owned by another runtime.  The single
  * 256x256-sized pair is the case that needs scratch memory at all (its rows are divided over
  * all SMs and the partial results are summed afterwards, see xcorr_workspace_bytes); this entry
- * point runs exactly that path with the partial results in an array that is part of the library
- * image instead of a caller-provided workspace.
+ * point runs the tile kernel's form of that path (not the tensor cores') with the partial results in an
+ * array that is part of the library image instead of a caller-provided workspace.
  *
  *  - The array holds xcorr_noalloc_scratch_bytes() = 32 MiB and exists on every GPU that loads the
  *    library, from load to process exit, whether this entry point is used or not.
@@ -265,9 +270,12 @@ XCORR_API int32_t xcorr_validate_input_size(int32_t mode, uint32_t rows, uint32_
                                             uint32_t n_left, uint32_t n_right);
 
 /* ---- FFT path ---------------------------------------------------------------------------
- * The same four modes through cuFFT: zero padding to 2*rows x 2*cols on the device, one batched
- * real-to-complex transform of all inputs, spectrum products left * conj(right), one batched
- * complex-to-real transform of all pairs, unpacking.  Stands in for the reference's
+ * The same four modes through transforms: left * conj(right) of the spectra.  In the normalized
+ * layout a pair whose half spectrum fits one SM is transformed, multiplied and transformed back by
+ * one block, at lengths of a power of two times at most one 3 and one 5 (a few large pairs excepted,
+ * which one block each would leave waiting).  All others, and the raw layout, go through cuFFT: zero padding to
+ * 2*rows x 2*cols on the device, one batched real-to-complex transform of all inputs, the spectrum
+ * products, one batched complex-to-real transform of all pairs, unpacking.  Stands in for the reference's
  * fft_original_alg_* / fft_reduced_transfer_* classes (one_to_one.hpp:888-1170,
  * one_to_many.hpp:502-780, n_to_mn.hpp:720-1000), fft_better_hadamard_alg_n_to_m
  * (n_to_m.hpp:647-800) and their kernels run_hadamard_original / run_hadamard_n_to_m_over_*
@@ -280,7 +288,7 @@ XCORR_API int32_t xcorr_validate_input_size(int32_t mode, uint32_t rows, uint32_
  * layout XCORR_FFT_RAW: `d_out` gets 2*rows x 2*cols per pair exactly as the inverse transform
  *   leaves it -- shift (sy, sx) at row sy mod 2*rows, column sx mod 2*cols, times 4*rows*cols:
  *   what the reference's fft classes hold in results() and write without --normalize.
- * The workspace (xcorr_fft_workspace_bytes) is required.  cuFFT plans are created on first use
+ * The workspace (xcorr_fft_workspace_bytes) is required.  Where cuFFT runs, its plans are created on first use
  * of a (device, size, batch) and cached; xcorr_fft_release_plans() destroys them.  A cached plan
  * owns one cuFFT work area: calls of the same shape on the same device must be ordered on one
  * stream (or otherwise not overlap on the GPU) -- unlike the direct entry points, which may run

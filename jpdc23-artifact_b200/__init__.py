@@ -213,7 +213,7 @@ def fft_out_shape(mode, rows, cols, n_left, n_right, layout="normalized"):
 def run_fft_device(mode, d_left: int, d_right: int, d_out: int, rows: int, cols: int, n_left: int,
                    n_right: int, layout="normalized", d_workspace: int = 0, workspace_bytes_: int = 0,
                    stream: int = 0) -> None:
-    """The cuFFT path on raw device addresses (asynchronous).  ``layout`` "normalized" gives the
+    """The FFT path on raw device addresses (asynchronous).  ``layout`` "normalized" gives the
     direct path's result layout, "raw" the 2*rows x 2*cols unnormalised inverse transforms."""
     check(lib().xcorr_fft_f32(_mode(mode), d_left, d_right, d_out, rows, cols, n_left, n_right,
                               FFT_LAYOUTS[layout], d_workspace or None, workspace_bytes_, stream or None))

@@ -642,8 +642,8 @@ bool tiny_auto(const xcorr_hints* h, const PairMap& pm, uint32_t rows, uint32_t 
 
 // Whether the automatic choice runs this call on the tensor cores: no hint asks for a plan of another
 // kernel, no plan less precise than the tile kernel's is considered, and the estimate beats the tile plan's by a
-// margin.  At this one none of 500 drawn shapes came out slower than the tile kernel, and 4 of 450 others by 4 % at
-// most (at 0.9: 10 of 500, by up to 12 %; the tile kernel's estimate is high where stream-K cuts few tasks).
+// margin.  At this one none of 500 drawn shapes came out slower than the tile kernel (at 0.9, with a fit to fewer plans,
+// 10 of 500 did, by up to 12 %: the tile kernel's estimate is high where stream-K cuts few tasks).
 constexpr double kTensorMargin = 0.865;
 bool tensor_auto(const xcorr_hints* h, const PairMap& pm, int H, int W, const DeviceInfo& dev, const TilePlan& tile,
                  int max_slices, TensorPlan* out) {

@@ -43,8 +43,8 @@
 // flight per SM every 7 clocks: 64 x 64 1 x 512 took 327 us), 4 and 16 matrices interleaved (fewer wraps, but all
 // warps wait for the one that writes: 32 x 32 32 x 64 88 us against 70), one sum of row totals h + small instead of two
 // (sparse operands off by 0.51..0.63 units, FFMAs 0.46..0.57).
-// Measured on B200 (us, tile kernel -> this one): 256 x 256 one pair 168 -> 107, 64 x 64 1 x 512 353 -> 153,
-// 32 x 32 32 x 64 102 -> 84, 48 x 48 16 x 2048 449 -> 296, 27 x 43 9 x 35 54 -> 33, 256 x 256 1 x 32 4655 -> 1904.
+// Measured on B200 (us, tile kernel -> this one): 256 x 256 one pair 168 -> 105, 64 x 64 1 x 512 353 -> 150,
+// 32 x 32 32 x 64 102 -> 82, 48 x 48 16 x 2048 449 -> 289, 27 x 43 9 x 35 54 -> 33, 256 x 256 1 x 32 4655 -> 1892.
 //
 // Roles of a block: the first 8 or 16 warps drain tensor memory into register sums and write results, three build the
 // Toeplitz rows, the last one issues the matrix products.
